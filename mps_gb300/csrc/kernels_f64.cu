@@ -1,9 +1,12 @@
 // Plain FP64 path: grouped block GEMM (one persistent launch over every sector GEMM of a
 // contraction) and the FP64 vector operations of the Krylov solver.
 //
-// GB300 runs FP64 at a small fraction of its FP32 rate, so the GEMM is a register-blocked
-// DFMA kernel whose only job is to keep the FP64 pipe busy: 64x64 output tile per CTA, 4x4
-// accumulators per thread, K staged through shared memory in steps of 16.
+// GB300 runs FP64 at a small fraction of its FP32 rate, so the tiled sector GEMMs run on the tensor
+// cores (kernels_f64tc.cu). The register-blocked DFMA kernel here (64x64 output tile per CTA, 4x4
+// accumulators per thread, K staged through shared memory in steps of 16) serves what must not
+// allocate scratch (mpsg_contract_noalloc), what finds no room for it, and K above 65536; the
+// thin kernels serve the MPO-sized contractions.
+#include "f64tc.hpp"
 #include "runtime.hpp"
 
 namespace mpsg {
@@ -302,11 +305,28 @@ void DevGemmPlan::build_host(const std::vector<GemmTask>& g, double flops_, Gemm
   ntiles = units[kTiled];
 }
 
-void DevGemmPlan::upload(const std::vector<GemmTask>& g, double flops_, cudaStream_t st) {
+void DevGemmPlan::upload(const std::vector<GemmTask>& g, double flops_, cudaStream_t st,
+                         bool tensor_cores) {
   release();
   stream = st;
   GemmTables t;
   build_host(g, flops_, t);
+  if (tensor_cores && count[kTiled]) {
+    std::vector<GemmTask> on, off;
+    for (const GemmTask& x : t.part[kTiled]) (f64tc::eligible(x) ? on : off).push_back(x);
+    if (!on.empty()) {
+      tc = std::make_shared<f64tc::Plan>();
+      tc->build(on, st);
+      // the other tiled tasks keep the FP64-pipe tables
+      GemmTables rest;
+      DevGemmPlan h;
+      h.build_host(off, 0, rest);
+      t.part[kTiled] = rest.part[kTiled];
+      t.prefix[kTiled] = rest.prefix[kTiled];
+      n = count[kTiled] = h.count[kTiled];
+      ntiles = units[kTiled] = h.units[kTiled];
+    }
+  }
   for (int q = 0; q < 3; ++q) {
     if (count[q] == 0) continue;
     const size_t bt = sizeof(GemmTask) * count[q], bp = sizeof(int64_t) * (count[q] + 1);
@@ -333,12 +353,17 @@ void DevGemmPlan::release() {
   d_prefix = nullptr;
   n = 0;
   ntiles = 0;
+  tc.reset();
 }
 
 void launch_gemm_f64(Context* ctx, const DevGemmPlan& p, const double* A, const double* B,
                      double* C) {
-  if (p.units[kTiled] + p.units[kRows] + p.units[kCols] == 0) return;
-  KernelTimer timer(ctx, kKindGemmF64, p.flops);
+  if (p.tc) f64tc::launch(ctx, *p.tc, A, B, C);
+  if (p.units[kTiled] + p.units[kRows] + p.units[kCols] == 0) {
+    if (p.tc) ctx->gemm_flops += p.flops;
+    return;
+  }
+  KernelTimer timer(ctx, kKindGemmF64, p.flops - (p.tc ? p.tc->flops() : 0.0));
   if (p.units[kTiled]) {
     int64_t grid = std::min<int64_t>(p.units[kTiled], (int64_t)ctx->num_sms * 4);
     gemm_f64_grouped_kernel<<<(unsigned)grid, 256, 0, ctx->stream>>>(

@@ -39,157 +39,52 @@
 #include <type_traits>
 
 #include "split.hpp"
+#include "tc5.cuh"
 
 namespace mpsg {
+namespace tc {
+
+typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
+                                  const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
+                                  const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
+                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+
+static EncodeTiledFn encode_fn() {
+  static std::atomic<EncodeTiledFn> fn{nullptr};
+  EncodeTiledFn f = fn.load();
+  if (!f) {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    MPSG_CUDA(cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000,
+                                               cudaEnableDefault, &q));
+    if (!p || q != cudaDriverEntryPointSuccess)
+      throw Error(kErrCuda, "cuTensorMapEncodeTiled is not available");
+    f = (EncodeTiledFn)p;
+    fn.store(f);
+  }
+  return f;
+}
+
+void make_slice_map(CUtensorMap* map, void* base, int64_t rows_total, int S, int box_rows,
+                    int row_len, int box_x) {
+  cuuint64_t gdim[3] = {(cuuint64_t)row_len, (cuuint64_t)rows_total, (cuuint64_t)S};
+  cuuint64_t gstride[2] = {2 * (cuuint64_t)row_len, (cuuint64_t)rows_total * 2 * row_len};
+  cuuint32_t box[3] = {(cuuint32_t)box_x, (cuuint32_t)box_rows, 1};
+  cuuint32_t es[3] = {1, 1, 1};
+  CUresult r = encode_fn()(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, base, gdim, gstride, box, es,
+                           CU_TENSOR_MAP_INTERLEAVE_NONE,
+                           box_x == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
+                           CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS)
+    throw Error(kErrCuda, "cuTensorMapEncodeTiled failed: " + std::to_string((int)r));
+}
+
+}  // namespace tc
+
 namespace split {
 
-// ------------------------------------------------------------------------------------------
-// device helpers (inline PTX)
-// ------------------------------------------------------------------------------------------
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return (uint32_t)__cvta_generic_to_shared(p);
-}
-
-__device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
-}
-
-__device__ __forceinline__ void mbar_expect_tx(uint64_t* bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)),
-               "r"(bytes)
-               : "memory");
-}
-
-__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
-}
-
-__device__ __forceinline__ uint32_t mbar_try_wait(uint64_t* bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.b32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(parity)
-      : "memory");
-  return ok;
-}
-
-constexpr long long kWaitCycles = 4000000000LL;  // about 2 s at the maximum SM clock
-
-// Bounded wait on a barrier phase; returns false (and raises the abort flag) on timeout or when
-// another role already aborted.
-__device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
-                                          int* err, int code) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const long long t0 = clock64();
-  for (;;) {
-    if (mbar_try_wait(bar, parity)) return true;
-    if (*abort_flag) return false;
-    if (clock64() - t0 > kWaitCycles) {
-      *abort_flag = 1;
-      atomicCAS(err, 0, code);
-      return false;
-    }
-  }
-}
-
-__device__ __forceinline__ void fence_barrier_init() {
-  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-}
-
-__device__ __forceinline__ void tc_fence_before() {
-  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-}
-
-__device__ __forceinline__ void tc_fence_after() {
-  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-}
-
-__device__ __forceinline__ void tmem_alloc(uint32_t* dst, uint32_t ncols) {
-  asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(
-                   smem_u32(dst)),
-               "r"(ncols)
-               : "memory");
-  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-}
-
-__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
-  asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols)
-               : "memory");
-}
-
-__device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc,
-                                          uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-  asm volatile(
-      "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-          smem_u32(bar))
-      : "memory");
-}
-
-__device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, uint64_t* bar,
-                                            int c0, int c1, int c2) {
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(smem_u32(dst)),
-      "l"((uint64_t)map), "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(bar))
-      : "memory");
-}
-
-// 32 consecutive FP32 columns of one TMEM lane per thread (shape 32x32b, 32 repetitions)
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
-        "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
-        "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]),
-        "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]), "=r"(v[24]), "=r"(v[25]),
-        "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
-// 16 consecutive FP32 columns of one TMEM lane per thread (shape 32x32b, 16 repetitions)
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
-        "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
-        "=r"(v[14]), "=r"(v[15])
-      : "r"(taddr));
-  asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-}
-
-// Shared-memory matrix descriptor: K-major operand tile, 128-byte swizzle, 8-row groups 1024 B
-// apart (stride byte offset), base 1024-byte aligned.
-__device__ __forceinline__ uint64_t sw128_desc(uint32_t saddr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);  // start address
-  d |= (uint64_t)1 << 16;                    // leading byte offset (unused for swizzled K-major)
-  d |= (uint64_t)(1024 >> 4) << 32;          // stride byte offset
-  d |= (uint64_t)1 << 46;                    // descriptor version
-  d |= (uint64_t)2 << 61;                    // 128-byte swizzle
-  return d;
-}
-
-// Instruction descriptor of kind::f16: FP32 accumulator, bf16 A and B, both K-major.
-__host__ __device__ constexpr uint32_t make_idesc(int M, int N) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) |
-         ((uint32_t)(M >> 4) << 24);
-}
+using namespace tc;
 
 // (hi + lo) * 2^E as FP64 using integer instructions only (hi, lo normal or zero FP32 values
 // with |lo| <= |hi|; a non-finite hi is returned as is).  Bits below 2^-62 of |hi| are
@@ -472,17 +367,6 @@ __global__ void __launch_bounds__(256) pack_slices_kernel(
 // ------------------------------------------------------------------------------------------
 // the GEMM kernel
 // ------------------------------------------------------------------------------------------
-// K-major tile with 64-byte swizzle (rows of 32 bf16), 8-row groups 512 B apart
-__device__ __forceinline__ uint64_t sw64_desc(uint32_t saddr) {
-  uint64_t d = 0;
-  d |= (uint64_t)((saddr & 0x3FFFFu) >> 4);  // start address
-  d |= (uint64_t)1 << 16;                    // leading byte offset (unused for swizzled K-major)
-  d |= (uint64_t)(512 >> 4) << 32;           // stride byte offset: 8 rows x 64 B
-  d |= (uint64_t)1 << 46;                    // descriptor version
-  d |= (uint64_t)4 << 61;                    // 64-byte swizzle
-  return d;
-}
-
 // Exact mode. The K step is 64 (128-byte swizzle) up to 3 slices; with 4..7 slices it is 32
 // (64-byte swizzle) so that a pipeline stage holding all S slices of both operands fits 2 to 4
 // times in shared memory. A chunk (the K range between exact FP32 flushes, exact_chunk) is a
@@ -511,12 +395,6 @@ struct Cfg {
   static constexpr int kThreads = 32 * (2 + kEpiWarps);
 };
 constexpr int kExactThreads = 576;  // Cfg<S, BN>::kThreads (launch bound of the exact kernel)
-
-// Static schedule shared by the three roles: the host sorts output tiles by decreasing K and the
-// CTAs deal them out in snake order (b, 2G-1-b, 2G+b, ...), which balances ragged sectors.
-__device__ __forceinline__ int64_t sched_pos(int64_t i, int G, int b) {
-  return i * G + ((i & 1) ? (G - 1 - b) : b);
-}
 
 // 18 warps put 5 warps on one SM sub-partition (16K registers), which caps a thread at 96
 // registers; the epilogue drains TMEM in 16-column pieces to stay close to that
@@ -942,40 +820,6 @@ __global__ void __launch_bounds__(192, 1) split_gemm_fast_kernel(
 // ------------------------------------------------------------------------------------------
 // host side
 // ------------------------------------------------------------------------------------------
-typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
-                                  const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                                  const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                  CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-static EncodeTiledFn encode_fn() {
-  static EncodeTiledFn fn = nullptr;
-  if (!fn) {
-    void* p = nullptr;
-    cudaDriverEntryPointQueryResult q;
-    MPSG_CUDA(cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &p, 12000,
-                                               cudaEnableDefault, &q));
-    if (!p || q != cudaDriverEntryPointSuccess)
-      throw Error(kErrCuda, "cuTensorMapEncodeTiled is not available");
-    fn = (EncodeTiledFn)p;
-  }
-  return fn;
-}
-
-// Packed operand [S][rows_total][64] bf16; box = box_x K-columns x box_rows rows of one slice.
-static void make_map(CUtensorMap* map, void* base, int64_t rows_total, int S, int box_rows,
-                     int box_x) {
-  cuuint64_t gdim[3] = {64, (cuuint64_t)rows_total, (cuuint64_t)S};
-  cuuint64_t gstride[2] = {128, (cuuint64_t)rows_total * 128};
-  cuuint32_t box[3] = {(cuuint32_t)box_x, (cuuint32_t)box_rows, 1};
-  cuuint32_t es[3] = {1, 1, 1};
-  CUresult r = encode_fn()(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, base, gdim, gstride, box, es,
-                           CU_TENSOR_MAP_INTERLEAVE_NONE,
-                           box_x == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
-                           CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) throw Error(kErrCuda, "cuTensorMapEncodeTiled failed: " + std::to_string((int)r));
-}
-
 int chunk_for(int S) { return exact_chunk(S); }
 
 }  // namespace split
@@ -1118,8 +962,8 @@ void SplitPlan::build(Context* ctx, const std::vector<GemmTask>& g, int S_, Tuni
   alloc((void**)&d_err, sizeof(int));
   zero(d_err, sizeof(int));
   const int box_x = (fast || S > 3) ? 32 : BK;  // K step of the kernel that reads the slices
-  make_map(&tmA, d_packA, std::max<int64_t>(rowsA, BM), S, BM, box_x);
-  make_map(&tmB, d_packB, std::max<int64_t>(rowsB, bn), S, bn, box_x);
+  make_slice_map(&tmA, d_packA, std::max<int64_t>(rowsA, BM), S, BM, 64, box_x);
+  make_slice_map(&tmB, d_packB, std::max<int64_t>(rowsB, bn), S, bn, 64, box_x);
 }
 
 void SplitPlan::release() {

@@ -37,8 +37,9 @@ void context_init(Context* ctx, int device) {
   uint64_t thr = UINT64_MAX;  // keep freed blocks cached in the pool
   MPSG_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &thr));
   MPSG_CUDA(cudaMalloc(&ctx->d_partials, sizeof(double) * (ctx->num_sms * 4 + 64)));
-  MPSG_CUDA(cudaMalloc(&ctx->d_copy_err, sizeof(int)));
-  MPSG_CUDA(cudaMemset(ctx->d_copy_err, 0, sizeof(int)));
+  MPSG_CUDA(cudaMalloc(&ctx->d_copy_err, 2 * sizeof(int)));
+  MPSG_CUDA(cudaMemset(ctx->d_copy_err, 0, 2 * sizeof(int)));
+  ctx->d_tc_err = ctx->d_copy_err + 1;
   MPSG_CUDA(cudaMallocHost(&ctx->h_pinned, sizeof(double) * Context::kPinnedDoubles));
   const char* dbg = std::getenv("MPSG_DEBUG_SYNC");
   ctx->debug_sync = dbg && dbg[0] == '1';

@@ -30,6 +30,9 @@ struct HeffPlans;
 namespace split {
 struct SplitPlan;
 }
+namespace f64tc {
+struct Plan;
+}
 
 // Stream-ordered device allocation.  Every buffer co-owns its context, so the context (stream,
 // caches) outlives the last tensor whatever order a caller releases handles in.
@@ -103,8 +106,11 @@ struct DevGemmPlan {
   std::vector<GemmTask> host;
   std::shared_ptr<split::SplitPlan> splitp[8];  // split-precision plans by slice count
   cudaStream_t stream = nullptr;  // tables are allocated and freed in this stream's order
+  std::shared_ptr<f64tc::Plan> tc;  // the tiled tasks that run on the tensor cores (FP64)
   size_t device_bytes() const;    // packed-slice scratch of the split plans (the bulk)
-  void upload(const std::vector<GemmTask>& g, double flops_, cudaStream_t st);
+  // tensor_cores = false keeps every task on the FP64 pipe (no scratch at launch).
+  void upload(const std::vector<GemmTask>& g, double flops_, cudaStream_t st,
+              bool tensor_cores = true);
   // Host half of upload: every field except the device pointers, plus the per-part tables.
   void build_host(const std::vector<GemmTask>& g, double flops_, GemmTables& t);
   void release();
@@ -177,6 +183,7 @@ struct Context : std::enable_shared_from_this<Context> {
   cudaStream_t stream = nullptr;
   double* d_partials = nullptr;   // reduction partials (one per CTA of a reduction launch)
   int* d_copy_err = nullptr;      // set by the TMA-staged copy kernel when a bounded wait expires
+  int* d_tc_err = nullptr;        // ... and by the FP64 tensor-core GEMM
   // small pinned host scratch: [0, 64) scalar results, [64, 64 + 3 * 128) the batched Lanczos
   static constexpr int kPinnedDoubles = 64 + 3 * 128;
   double* h_pinned = nullptr;

@@ -1,0 +1,85 @@
+"""The FP64 block GEMM on the tensor cores against extended-precision products, and against the
+FP64-pipe kernels (which the allocation-free contraction keeps) for values outside its range."""
+import numpy as np
+import pytest
+
+import mps_gb300 as mg
+from mps_gb300._lib import call, i32arr
+
+pytestmark = pytest.mark.gpu
+
+# edges of the 128 x 64 tile, of the 32-wide K step, of the 256-wide chunk between drains, both
+# orientations (few rows, few columns) and several blocks of different size in one launch
+SHAPES = [((33,), (33,), (33,)), ((128,), (64,), (32,)), ((129,), (65,), (257,)),
+          ((40,), (513,), (256,)), ((600,), (41,), (255,)), ((1,), (200,), (40,)),
+          ((64, 7, 130), (257, 50, 40), (33, 1, 1031))]
+
+
+def pair(ms, ns, ks, seed=3):
+    rng = np.random.Generator(np.random.Philox(seed))
+    V, K, N = (mg.U1Space(*enumerate(x)) for x in (ms, ks, ns))
+    a = [rng.standard_normal((m, k)) for m, k in zip(ms, ks)]
+    b = [rng.standard_normal((k, n)) for k, n in zip(ks, ns)]
+    return (V, K, N), a, b
+
+
+def product(spaces, a, b, pipe=False):
+    V, K, N = spaces
+    A = mg.from_flat(0, (V, mg.dual(K)), np.concatenate([x.ravel(order="F") for x in a]))
+    B = mg.from_flat(0, (K, mg.dual(N)), np.concatenate([x.ravel(order="F") for x in b]))
+    if pipe:
+        C = mg.zeros(0, (V, mg.dual(N)))
+        call("mpsg_contract_noalloc", A.ctx.handle, A.handle, i32arr((1, -1)), B.handle,
+             i32arr((-1, 2)), C.handle)
+    else:
+        C = mg.contract(A, (1, -1), B, (-1, 2), precision=0)
+    f, out, p = C.to_flat(), [], 0
+    for x, y in zip(a, b):
+        n = x.shape[0] * y.shape[1]
+        out.append(f[p:p + n].reshape((x.shape[0], y.shape[1]), order="F"))
+        p += n
+    return out
+
+
+@pytest.mark.parametrize("ms,ns,ks", SHAPES)
+def test_rounded_once(ms, ns, ks):
+    """Rounding the exact sum is at most 2^-53 of it; the digits left out add below 2^-57 of the
+    result's norm for normal data, so a quarter more covers both."""
+    spaces, a, b = pair(ms, ns, ks)
+    rng = np.random.default_rng(1)
+    for x, y, g in zip(a, b, product(spaces, a, b)):
+        rows = np.sort(rng.choice(x.shape[0], min(x.shape[0], 24), replace=False))
+        want = x[rows].astype(np.longdouble) @ y.astype(np.longdouble)
+        err = np.linalg.norm((g[rows] - want).astype(float))
+        assert err <= 1.25 * 2.0 ** -53 * np.linalg.norm(want.astype(float))
+
+
+@pytest.mark.parametrize("ms,ns,ks", SHAPES)
+def test_integers_exact(ms, ns, ks):
+    spaces, a, b = pair(ms, ns, ks)
+    a, b = [np.rint(50 * x) for x in a], [np.rint(50 * x) for x in b]
+    for x, y, g in zip(a, b, product(spaces, a, b)):
+        assert np.array_equal(g, x @ y)
+
+
+def test_values_outside_the_sliced_range():
+    """NaN, infinities, subnormals and rows of extreme magnitude give what the FP64 pipe gives;
+    scaled ordinary rows and columns keep their relative accuracy."""
+    spaces, (a,), (b,) = pair((150,), (90,), (50,))
+    a[3, 4], a[12, 7] = np.inf, np.nan
+    a[9, :], a[10], a[11], a[13] = 0.0, a[10] * 1e-200, a[11] * 1e200, 5e-324
+    b[2, 8], b[:, 6] = -np.inf, 0.0
+    b[:, 5], b[:, 9], b[:, 10] = b[:, 5] * 1e-300, b[:, 9] * 1e250, b[:, 10] * 1e-90
+    (g,), (h,) = product(spaces, [a], [b]), product(spaces, [a], [b], pipe=True)
+    assert np.array_equal(np.isnan(g), np.isnan(h))
+    assert np.array_equal(g[np.isinf(h)], h[np.isinf(h)])
+    odd = np.zeros(g.shape, bool)
+    odd[[3, 10, 11, 12, 13]], odd[:, [5, 8, 9]] = True, True
+    same = odd & np.isfinite(h)
+    assert np.array_equal(g[same], h[same])  # the same FMA chain
+    assert np.all(g[9, np.isfinite(h[9])] == 0.0)
+    rest = ~odd & np.isfinite(h)
+    with np.errstate(all="ignore"):
+        scale = np.abs(a).max(axis=1)[:, None] * np.abs(b).max(axis=0)[None, :]
+    # K FMA roundings of at most 2^-53 of partial sums below K times the scale
+    assert np.all(np.abs(g[rest] - h[rest]) <= 50 * 50 * 2.0 ** -53 * scale[rest])
