@@ -306,17 +306,21 @@ void DevGemmPlan::build_host(const std::vector<GemmTask>& g, double flops_, Gemm
 }
 
 void DevGemmPlan::upload(const std::vector<GemmTask>& g, double flops_, cudaStream_t st,
-                         bool tensor_cores) {
+                         int num_sms) {
   release();
   stream = st;
   GemmTables t;
   build_host(g, flops_, t);
-  if (tensor_cores && count[kTiled]) {
-    std::vector<GemmTask> on, off;
-    for (const GemmTask& x : t.part[kTiled]) (f64tc::eligible(x) ? on : off).push_back(x);
+  if (num_sms > 0 && count[kTiled]) {
+    std::vector<f64tc::Task> on;
+    std::vector<GemmTask> off;
+    for (const GemmTask& x : t.part[kTiled]) {
+      if (f64tc::eligible(x)) on.push_back(f64tc::Task{x});
+      else off.push_back(x);
+    }
     if (!on.empty()) {
       tc = std::make_shared<f64tc::Plan>();
-      tc->build(on, st);
+      tc->build(on, num_sms, st);
       // the other tiled tasks keep the FP64-pipe tables
       GemmTables rest;
       DevGemmPlan h;

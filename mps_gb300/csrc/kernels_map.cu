@@ -1,0 +1,375 @@
+// Sector GEMMs of a contraction on the FP64 pipe, reading the operand tensors and writing the result
+// tensor in place through index maps (contract_map.hpp): the element-per-thread kernel for small
+// contractions and the thin kernel for MPO-sized ones. The large sector GEMMs take the same maps
+// into the tensor-core kernels (kernels_f64tc.cu).
+#include <algorithm>
+
+#include "copy_decode.hpp"
+#include "direct.hpp"
+
+namespace mpsg {
+
+namespace {
+
+struct BlockRegs {
+  int64_t base;
+  int rs0, rs1, rs2, cs0, cs1, cs2;
+};
+
+__device__ __forceinline__ BlockRegs load_block(const MapBlock* b) {
+  const int4* p = reinterpret_cast<const int4*>(b);
+  const int4 x = __ldg(p), y = __ldg(p + 1);
+  return BlockRegs{(int64_t)(((unsigned long long)(unsigned)x.y << 32) | (unsigned)x.x),
+                   x.z, x.w, y.x, y.y, y.z, y.w};
+}
+
+__device__ __forceinline__ int64_t row_part(const BlockRegs& b, const int4& e) {
+  return b.base + (e.y * b.rs0 + e.z * b.rs1 + e.w * b.rs2);
+}
+
+__device__ __forceinline__ int col_part(const BlockRegs& b, const int4& e) {
+  return e.y * b.cs0 + e.z * b.cs1 + e.w * b.cs2;
+}
+
+// One thread per result element, every sector GEMM of a small contraction in one launch. Bound by
+// latency: the chain of a thread is K dependent FMAs behind prefetched loads, so what counts is
+// that the elements spread over the whole chip (a 64 x 64 tile kernel keeps them on a few SMs, each
+// at 2 FMAs per cycle) and that nothing runs before or after it. Measured, the four contractions of
+// a chi = 48 two-site H_eff: 4 launches of 7.3 us against 19 of 205 us in all.
+__global__ void __launch_bounds__(128) contract_small_kernel(
+    const SmallProblem* __restrict__ probs, int nprob, int64_t total,
+    const int2* __restrict__ kcombos, const AxisEntry* __restrict__ axes,
+    const MapBlock* __restrict__ blocks, const double* __restrict__ A,
+    const double* __restrict__ B, double* __restrict__ C) {
+  const int4* ax = reinterpret_cast<const int4*>(axes);
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total;
+       e += (int64_t)gridDim.x * blockDim.x) {
+    int lo = 0, hi = nprob - 1;
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) >> 1;
+      if (__ldg(&probs[mid].first) <= e) lo = mid;
+      else hi = mid - 1;
+    }
+    const SmallProblem& P = probs[lo];
+    const uint32_t lt = (uint32_t)(e - P.first);
+    const uint32_t j = lt / (uint32_t)P.M, i = lt - j * (uint32_t)P.M;
+    const int4 me = __ldg(ax + P.axM + i), ne = __ldg(ax + P.axN + j);
+    const int nkc = P.nkc;
+    const MapBlock* ta = blocks + P.blkA + (me.x & kComboMask) * nkc;
+    const MapBlock* tb = blocks + P.blkB + (ne.x & kComboMask) * nkc;
+    const int4* ke = ax + P.axK;
+    double acc = 0.0;
+    for (int c = 0; c < nkc; ++c) {
+      const int2 kc = __ldg(kcombos + P.kc0 + c);
+      const BlockRegs ba = load_block(ta + c), bb = load_block(tb + c);
+      const double* pa = A + row_part(ba, me);
+      const double* pb = B + row_part(bb, ne);
+#pragma unroll 8
+      for (int k = 0; k < kc.y; ++k) {
+        const int4 x = __ldg(ke + kc.x + k);
+        acc = fma(__ldg(pa + col_part(ba, x)), __ldg(pb + col_part(bb, x)), acc);
+      }
+    }
+    const BlockRegs bc = load_block(blocks + P.blkC + (me.x & kComboMask) * P.nnc + (ne.x & kComboMask));
+    C[row_part(bc, me) + col_part(bc, ne)] = acc;
+  }
+}
+
+// Thin sector GEMMs (the MPO steps: T and K at most 32): a thread owns indices of the long axis,
+// reads the K elements of each and writes T results, coalesced along the long axis; the thin
+// operand sits in shared memory. Bound by the FP64 pipe (2 FMAs per SM and cycle) and HBM about
+// equally for the XXZ MPO (K = T = 4), so FMAs with an exact zero of the thin operand are skipped
+// (12 of its 34 allowed entries are not zero), a first term of 1.0 x is taken as x, and
+// several rows are in flight per thread. A row with a non-finite element does every FMA, as 0 x Inf
+// must give NaN. Measured, the MPO steps of a two-site H_eff with the copies that they replace:
+// chi = 2048 2 x 72 us (before 434), chi = 517 2 x 12 us (93).
+struct ThinShared {
+  ThinOffset o[2 * kThinMax];    // K of the long operand, T of the output
+  uint32_t mask[kThinMax];       // nonzero entries of a thin index
+  uint32_t one[kThinMax];        // its lowest nonzero entry if that is exactly 1.0
+  double b[kThinMax * kThinMax];  // [thin][k]
+};
+
+// x as fma(x, 1.0, 0.0) gives it: -0.0 becomes 0.0
+__device__ __forceinline__ double times_one(double x) {
+  const long long b = __double_as_longlong(x);
+  return __longlong_as_double(b == (long long)(1ull << 63) ? 0 : b);
+}
+
+// ROWS groups of 32 rows, one row of each per lane, from `row` on (all groups below u.count begin
+// inside the unit).
+template <int KMAX, int ROWS>
+__device__ __forceinline__ void thin_rows(const ThinShared& s, const ThinUnit& u, int row,
+                                          const double* __restrict__ X, double* __restrict__ C) {
+  const int K = u.K;
+  int i0[ROWS], i1[ROWS], i2[ROWS];
+  bool in[ROWS];
+  double a[ROWS][KMAX];
+#pragma unroll
+  for (int y = 0; y < ROWS; ++y) {
+    in[y] = row + 32 * y < u.count;
+    const uint32_t q = (uint32_t)(u.start + (in[y] ? row + 32 * y : 0));
+    const uint32_t q0 = fdiv(q, u.m0, u.s0);
+    i0[y] = (int)(q - q0 * u.d0);
+    i2[y] = (int)fdiv(q0, u.m1, u.s1);
+    i1[y] = (int)(q0 - (uint32_t)i2[y] * u.d1);
+  }
+#pragma unroll
+  for (int k = 0; k < KMAX; ++k) {
+    if (k < K) {
+      const ThinOffset o = s.o[k];
+#pragma unroll
+      for (int y = 0; y < ROWS; ++y)
+        a[y][k] = __ldg(X + o.off + (i0[y] * o.rs0 + i1[y] * o.rs1 + i2[y] * o.rs2));
+    } else {
+#pragma unroll
+      for (int y = 0; y < ROWS; ++y) a[y][k] = 0.0;
+    }
+  }
+  int bad = 0;
+#pragma unroll
+  for (int y = 0; y < ROWS; ++y)
+#pragma unroll
+    for (int k = 0; k < KMAX; ++k) bad |= (__double2hiint(a[y][k]) & 0x7ff00000) == 0x7ff00000;
+  for (int t = 0; t < u.T; ++t) {
+    const uint32_t mask = bad ? (K == 32 ? 0xffffffffu : (1u << K) - 1u) : s.mask[t];
+    const uint32_t one = bad ? 0u : s.one[t];
+    double acc[ROWS];
+#pragma unroll
+    for (int y = 0; y < ROWS; ++y) acc[y] = 0.0;
+#pragma unroll
+    for (int k = 0; k < KMAX; ++k) {
+      if (one >> k & 1u) {
+#pragma unroll
+        for (int y = 0; y < ROWS; ++y) acc[y] = times_one(a[y][k]);
+      } else if (mask >> k & 1u) {
+        const double b = s.b[t * K + k];
+#pragma unroll
+        for (int y = 0; y < ROWS; ++y) acc[y] = fma(a[y][k], b, acc[y]);
+      }
+    }
+    const ThinOffset o = s.o[K + t];
+#pragma unroll
+    for (int y = 0; y < ROWS; ++y)
+      if (in[y]) C[o.off + (i0[y] * o.rs0 + i1[y] * o.rs1 + i2[y] * o.rs2)] = acc[y];
+  }
+}
+
+template <int KMAX, int ROWS>
+__global__ void __launch_bounds__(256) contract_thin_kernel(
+    const ThinUnit* __restrict__ units, int nunits, const ThinOffset* __restrict__ offs,
+    const int64_t* __restrict__ vals, const double* __restrict__ A, const double* __restrict__ B,
+    double* __restrict__ C) {
+  __shared__ ThinShared s;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int it = blockIdx.x; it < nunits; it += gridDim.x) {
+    const ThinUnit u = units[it];
+    const double* L = u.longB ? B : A;
+    const double* S = u.longB ? A : B;
+    __syncthreads();  // the previous unit has been read
+    if (threadIdx.x < u.K + u.T) s.o[threadIdx.x] = offs[u.offs + threadIdx.x];
+    for (int x = threadIdx.x; x < u.T * u.K; x += blockDim.x)
+      s.b[x] = __ldg(S + __ldg(vals + u.vals + x));
+    __syncthreads();
+    if (threadIdx.x < u.T) {
+      const double* b = s.b + threadIdx.x * u.K;
+      uint32_t m = 0;
+      for (int k = 0; k < u.K; ++k) m |= (uint32_t)(__double_as_longlong(b[k]) << 1 != 0) << k;
+      s.mask[threadIdx.x] = m;
+      s.one[threadIdx.x] =
+          m && __double_as_longlong(b[__ffs(m) - 1]) == 0x3ff0000000000000ll ? m & (0u - m) : 0u;
+    }
+    __syncthreads();
+    // rows of a warp are 32 ROWS in a row; at the end of the unit the warps take 32 each
+    const int full = u.count / (256 * ROWS) * (256 * ROWS);
+    for (int r = 32 * ROWS * warp; r < full; r += 256 * ROWS)
+      thin_rows<KMAX, ROWS>(s, u, r + lane, L, C);
+    if (ROWS > 1)
+      for (int r = full + 32 * warp; r < u.count; r += 256) thin_rows<KMAX, 1>(s, u, r + lane, L, C);
+    else if (full + 32 * warp < u.count)
+      thin_rows<KMAX, ROWS>(s, u, full + 32 * warp + lane, L, C);
+  }
+}
+
+// FMAs of a contraction that stays element-per-thread: 2^21 take the FP64 pipes of 152 SMs 3.5 us when
+// spread evenly, the tensor-core pair of launches about 20 us for anything.
+constexpr int64_t kSmallFma = 1 << 21;
+constexpr int64_t kSmallAxes = 1 << 16;  // ... and its axis entries (16 bytes each)
+constexpr int64_t kSmallK = 256;
+// Longest thin sector GEMM that joins the tensor-core launch when the contraction has one anyway: a
+// few padded tiles there, against a launch of its own (22 to 30 us for the edge charges of a
+// chi = 2048 environment, whose 32 x 32 FMAs per row sit on a few SMs).
+constexpr int64_t kTiledThin = 4096;
+
+}  // namespace
+
+void plan_direct(const std::vector<MapProblem>& map, const std::vector<GemmTask>& gemms,
+                 int num_sms, DirectTables& t) {
+  int64_t fma = 0, axes = 0, kmax = 0, thin_rows = 0;
+  bool tiled = false;
+  for (const MapProblem& q : map) {
+    fma += q.M * q.N * std::max<int64_t>(q.K, 1);
+    axes += q.M + q.N + q.K;
+    kmax = std::max(kmax, q.K);
+    if (q.K <= kThinMax && std::min(q.M, q.N) <= kThinMax) thin_rows += std::max(q.M, q.N);
+    else tiled = true;
+  }
+  const bool small = fma <= kSmallFma && axes <= kSmallAxes && kmax <= kSmallK;
+  // rows per thin unit: about eight units per SM, so that staging a unit's tables is shared by
+  // many rows and the last wave is short
+  const int64_t unit = std::min<int64_t>(
+      2048, std::max<int64_t>(256, (thin_rows / (8 * num_sms) + 255) / 256 * 256));
+  for (size_t p = 0; p < map.size(); ++p) {
+    const MapProblem& q = map[p];
+    auto axis = [&](const std::vector<AxisCombo>& c) {
+      const int32_t at = (int32_t)t.axes.size();
+      append_axis(c, t.axes);
+      return at;
+    };
+    auto table = [&](const std::vector<MapBlock>& b) {
+      const int32_t at = (int32_t)t.blocks.size();
+      t.blocks.insert(t.blocks.end(), b.begin(), b.end());
+      return at;
+    };
+    if (small) {
+      SmallProblem s;
+      s.first = t.elements;
+      s.M = (int32_t)q.M;
+      s.N = (int32_t)q.N;
+      s.axM = axis(q.m);
+      s.axN = axis(q.n);
+      s.axK = axis(q.k);
+      s.kc0 = (int32_t)t.kcombos.size();
+      s.nkc = (int32_t)q.k.size();
+      s.nnc = (int32_t)q.n.size();
+      for (const AxisCombo& c : q.k) t.kcombos.push_back(make_int2(c.start, c.count));
+      s.blkA = table(q.A);
+      s.blkB = table(q.B);
+      s.blkC = table(q.C);
+      t.elements += q.M * q.N;
+      t.small.push_back(s);
+    } else if (q.K <= kThinMax && std::min(q.M, q.N) <= kThinMax &&
+               !(tiled && std::max(q.M, q.N) <= kTiledThin)) {
+      const bool longB = q.M < q.N;
+      const auto &lc = longB ? q.n : q.m, &tc = longB ? q.m : q.n;
+      const auto &tl = longB ? q.B : q.A, &tt = longB ? q.A : q.B;
+      std::vector<AxisEntry> te, ke;
+      append_axis(tc, te);
+      append_axis(q.k, ke);
+      auto at = [](const AxisEntry& e, const int32_t* str) {
+        int64_t o = 0;
+        for (int d = 0; d < kMapLegs; ++d) o += (int64_t)e.i[d] * str[d];
+        return o;
+      };
+      const int32_t vals = (int32_t)t.vals.size();
+      for (const AxisEntry& x : te)
+        for (const AxisEntry& y : ke) {
+          const MapBlock& b = tt[(x.combo_run & kComboMask) * q.k.size() +
+                                 (y.combo_run & kComboMask)];
+          t.vals.push_back(b.base + at(x, b.rs) + at(y, b.cs));
+        }
+      for (size_t i = 0; i < lc.size(); ++i) {
+        const int32_t offs = (int32_t)t.offs.size();
+        for (const AxisEntry& y : ke) {
+          const MapBlock& b = tl[i * q.k.size() + (y.combo_run & kComboMask)];
+          t.offs.push_back(ThinOffset{b.base + at(y, b.cs), b.rs[0], b.rs[1], b.rs[2], 0});
+        }
+        for (const AxisEntry& x : te) {
+          const size_t j = x.combo_run & kComboMask;
+          const MapBlock& b = longB ? q.C[j * lc.size() + i] : q.C[i * tc.size() + j];
+          const int32_t *row = longB ? b.cs : b.rs, *thin = longB ? b.rs : b.cs;
+          t.offs.push_back(ThinOffset{b.base + at(x, thin), row[0], row[1], row[2], 0});
+        }
+        for (int64_t r = 0; r < lc[i].count; r += unit) {
+          ThinUnit u{};
+          u.T = (int32_t)te.size();
+          u.K = (int32_t)ke.size();
+          u.longB = longB;
+          u.offs = offs;
+          u.vals = vals;
+          u.start = (int32_t)r;
+          u.count = (int32_t)std::min<int64_t>(unit, lc[i].count - r);
+          u.d0 = (uint32_t)lc[i].d[0];
+          u.d1 = (uint32_t)lc[i].d[1];
+          magic_u31(u.d0, u.m0, u.s0);
+          magic_u31(u.d1, u.m1, u.s1);
+          t.units.push_back(u);
+        }
+      }
+    } else {
+      t.tiled.push_back(f64tc::Task{gemms[p], &q});
+    }
+  }
+  std::stable_sort(t.units.begin(), t.units.end(),
+                   [](const ThinUnit& a, const ThinUnit& b) { return a.count > b.count; });
+}
+
+bool DirectPlan::build(const ContractPlan& p, const TensorMeta& A, const TensorMeta& B,
+                       int num_sms, cudaStream_t st) {
+  const std::vector<MapProblem> map = build_contract_map(p, A, B);
+  if (map.empty()) return false;
+  DirectTables t;
+  plan_direct(map, p.mm.gemms, num_sms, t);
+  for (const auto& x : t.tiled)
+    if (!f64tc::eligible(x.g)) return false;
+  // nothing to save: the operands and the result are the fused matrices already
+  if (!t.tiled.empty() && p.fa.identity && p.fb.identity && p.split.identity) return false;
+  stream = st;
+  flops = p.flops;
+  for (const auto& x : t.tiled) tc_flops += 2.0 * x.g.M * x.g.N * x.g.K;
+  TableImage img;
+  const size_t os = img.add(t.small), ok = img.add(t.kcombos),
+               ou = img.add(t.units), of = img.add(t.offs), ov = img.add(t.vals), oa = img.add(t.axes), ob = img.add(t.blocks);
+  d_tables = img.upload(st);
+  d_small = (SmallProblem*)(d_tables + os);
+  d_kcombos = (int2*)(d_tables + ok);
+  d_units = (ThinUnit*)(d_tables + ou);
+  d_offs = (ThinOffset*)(d_tables + of);
+  d_vals = (int64_t*)(d_tables + ov);
+  d_axes = (AxisEntry*)(d_tables + oa);
+  d_blocks = (MapBlock*)(d_tables + ob);
+  nsmall = (int)t.small.size();
+  nunits = (int)t.units.size();
+  elements = t.elements;
+  for (const ThinUnit& x : t.units) thin_k = std::max(thin_k, x.K);
+  if (!t.tiled.empty()) {
+    tc = std::make_unique<f64tc::Plan>();
+    tc->build(t.tiled, num_sms, st);
+  }
+  return true;
+}
+
+DirectPlan::~DirectPlan() {
+  if (d_tables) cudaFreeAsync(d_tables, stream);
+}
+
+bool launch_direct(Context* ctx, DirectPlan& p, const double* A, const double* B, double* C) {
+  cudaStream_t st = ctx->stream;
+  if (p.tc && !f64tc::launch(ctx, *p.tc, A, B, C)) return false;
+  if (p.elements || p.nunits) {
+    KernelTimer timer(ctx, kKindGemmF64, p.flops - p.tc_flops);
+    if (p.elements) {
+      const int64_t grid = std::min<int64_t>((p.elements + 127) / 128, (int64_t)ctx->num_sms * 16);
+      contract_small_kernel<<<(unsigned)grid, 128, 0, st>>>(p.d_small, p.nsmall, p.elements,
+                                                           p.d_kcombos, p.d_axes, p.d_blocks, A,
+                                                           B, C);
+      MPSG_CUDA(cudaGetLastError());
+      ctx->kernel_launches++;
+    }
+    if (p.nunits) {
+      // rows in flight per thread by the longest K, within 64 (K <= 8) or 128 registers
+      auto kern = p.thin_k <= 4   ? contract_thin_kernel<4, 4>
+                  : p.thin_k <= 8 ? contract_thin_kernel<8, 2>
+                  : p.thin_k <= 16 ? contract_thin_kernel<16, 1>
+                                   : contract_thin_kernel<32, 1>;
+      const int grid = std::min(p.nunits, ctx->num_sms * 8);
+      kern<<<grid, 256, 0, st>>>(p.d_units, p.nunits, p.d_offs, p.d_vals, A, B, C);
+      MPSG_CUDA(cudaGetLastError());
+      ctx->kernel_launches++;
+    }
+  }
+  ctx->gemm_flops += p.flops;
+  return true;
+}
+
+}  // namespace mpsg

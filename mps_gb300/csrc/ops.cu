@@ -3,6 +3,7 @@
 #include <algorithm>
 #include <sstream>
 
+#include "direct.hpp"
 #include "ops.hpp"
 #include "split.hpp"
 
@@ -254,7 +255,7 @@ DeviceTensor matmul(Context* ctx, const DeviceTensor& a, const DeviceTensor& b, 
   if (!g) {
     MatmulPlan mp = plan_matmul(a.meta, b.meta);
     g = std::make_shared<DevGemmPlan>();
-    g->upload(mp.gemms, mp.flops, ctx->stream);
+    g->upload(mp.gemms, mp.flops, ctx->stream, ctx->num_sms);
     ctx->matmul_cache.put(key, g);
   }
   DeviceTensor t;
@@ -276,18 +277,35 @@ std::shared_ptr<DevContract> get_contract_plan(Context* ctx, const TensorMeta& A
   if (auto hit = ctx->contract_cache.get(key)) return hit;
   auto p = std::make_shared<DevContract>();
   p->host = plan_contract(A, idxA, B, idxB);
-  if (!p->host->scalar) {
-    p->fa.upload(p->host->fa.tasks, p->host->fa.identity, ctx->stream);
-    p->fb.upload(p->host->fb.tasks, p->host->fb.identity, ctx->stream);
-    p->mm.upload(p->host->mm.gemms, p->host->mm.flops, ctx->stream);
-    p->split.upload(p->host->split.tasks, p->host->split.identity, ctx->stream);
-  }
+  p->metaA = A;
+  p->metaB = B;
   ctx->contract_cache.put(key, p);
   return p;
 }
 
+// The fused path's tables (copies in, sector GEMMs, split): what the split-precision products, the
+// operator folds and FP64 contractions without an index map run on.
+static void ensure_fused(Context* ctx, DevContract& p) {
+  if (p.fused) return;
+  p.fa.upload(p.host->fa.tasks, p.host->fa.identity, ctx->stream);
+  p.fb.upload(p.host->fb.tasks, p.host->fb.identity, ctx->stream);
+  p.mm.upload(p.host->mm.gemms, p.host->mm.flops, ctx->stream, ctx->num_sms);
+  p.split.upload(p.host->split.tasks, p.host->split.identity, ctx->stream);
+  p.fused = true;
+}
+
+static DirectPlan* direct_plan(Context* ctx, DevContract& p) {
+  if (!p.direct_tried) {
+    auto d = std::make_shared<DirectPlan>();
+    if (d->build(*p.host, p.metaA, p.metaB, ctx->num_sms, ctx->stream)) p.direct = d;
+    p.direct_tried = true;
+  }
+  return p.direct.get();
+}
+
 std::shared_ptr<Buffer> contract_gemm(Context* ctx, DevContract& p, const DeviceTensor& a,
                                       const DeviceTensor& b, int precision) {
+  ensure_fused(ctx, p);
   std::shared_ptr<Buffer> fa, fb;
   const double* pa = a.data();
   const double* pb = b.data();
@@ -332,10 +350,15 @@ DeviceTensor contract(Context* ctx, const DeviceTensor& a, const std::vector<int
     if (scalar) *scalar = s;
     return DeviceTensor();
   }
-  std::shared_ptr<Buffer> fc = contract_gemm(ctx, *p, a, b, precision);
   DeviceTensor t;
   t.ctx = ctx;
   t.meta = p->host->split.out;
+  if (DirectPlan* d = precision == 0 ? direct_plan(ctx, *p) : nullptr) {
+    t.buf = alloc_buffer(ctx, t.meta.total);
+    if (launch_direct(ctx, *d, a.data(), b.data(), t.data())) return t;
+    t.buf.reset();
+  }
+  std::shared_ptr<Buffer> fc = contract_gemm(ctx, *p, a, b, precision);
   if (p->split.identity) {
     t.buf = fc;
   } else {
@@ -477,6 +500,7 @@ static std::shared_ptr<DevContract> private_contract_plan(Context* ctx, const Te
   p->fb.upload(p->host->fb.tasks, p->host->fb.identity, ctx->stream);
   p->mm.upload(p->host->mm.gemms, p->host->mm.flops, ctx->stream);
   p->split.upload(p->host->split.tasks, p->host->split.identity, ctx->stream);
+  p->fused = true;
   return p;
 }
 

@@ -4,6 +4,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <array>
 #include <atomic>
 #include <list>
@@ -108,18 +109,24 @@ struct DevGemmPlan {
   cudaStream_t stream = nullptr;  // tables are allocated and freed in this stream's order
   std::shared_ptr<f64tc::Plan> tc;  // the tiled tasks that run on the tensor cores (FP64)
   size_t device_bytes() const;    // packed-slice scratch of the split plans (the bulk)
-  // tensor_cores = false keeps every task on the FP64 pipe (no scratch at launch).
-  void upload(const std::vector<GemmTask>& g, double flops_, cudaStream_t st,
-              bool tensor_cores = true);
+  // num_sms > 0: the tiled tasks run on the tensor cores of that many SMs; 0 keeps every task on
+  // the FP64 pipe (no scratch at launch).
+  void upload(const std::vector<GemmTask>& g, double flops_, cudaStream_t st, int num_sms = 0);
   // Host half of upload: every field except the device pointers, plus the per-part tables.
   void build_host(const std::vector<GemmTask>& g, double flops_, GemmTables& t);
   void release();
 };
 
+struct DirectPlan;
+
 struct DevContract {
   std::shared_ptr<ContractPlan> host;
+  TensorMeta metaA, metaB;             // operand structures, to build the pieces below on first use
   DevCopyPlan fa, fb, split;
   DevGemmPlan mm;
+  bool fused = false;                  // fa, fb, split and mm are on the device
+  bool direct_tried = false;
+  std::shared_ptr<DirectPlan> direct;  // FP64 without fused copies (null: not for this structure)
   size_t device_bytes() const { return mm.device_bytes(); }
   ~DevContract();
 };
@@ -264,6 +271,29 @@ void set_smem_limit_once(Context* ctx, std::once_flag (&flags)[kMaxDevices], Ker
       throw Error(kErrCuda, std::string("cudaFuncSetAttribute: ") + cudaGetErrorString(e));
   });
 }
+
+inline size_t round256(size_t n) { return (n + 255) & ~size_t(255); }
+
+// Host image of several plan tables, placed on the device in one allocation and one copy (both in
+// the stream's order; a pageable source is staged before the copy returns).
+struct TableImage {
+  std::vector<unsigned char> bytes;
+  template <class T>
+  size_t add(const std::vector<T>& v) {  // offset of the table
+    const size_t at = bytes.size();
+    const unsigned char* p = (const unsigned char*)v.data();
+    bytes.insert(bytes.end(), p, p + sizeof(T) * v.size());
+    bytes.resize(round256(bytes.size()));
+    return at;
+  }
+  unsigned char* upload(cudaStream_t st) const {
+    unsigned char* d = nullptr;
+    MPSG_CUDA(cudaMallocAsync((void**)&d, std::max<size_t>(bytes.size(), 16), st));
+    if (!bytes.empty())
+      MPSG_CUDA(cudaMemcpyAsync(d, bytes.data(), bytes.size(), cudaMemcpyHostToDevice, st));
+    return d;
+  }
+};
 
 // ---- kernel launchers (kernels_*.cu) ----
 void launch_copy(Context* ctx, const DevCopyPlan& p, const double* src, double* dst);

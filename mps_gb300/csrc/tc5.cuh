@@ -99,6 +99,43 @@ __device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t adesc, uint6
       : "memory");
 }
 
+// The same with a hint for the A collector buffer: consecutive MMAs on one A tile read it from shared
+// memory once (kFillA on the first, kUseA, kLastA on the last).
+enum { kDiscardA = 0, kFillA = 1, kUseA = 2, kLastA = 3 };
+template <int OP>
+__device__ __forceinline__ void umma_bf16_a(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc,
+                                            uint32_t idesc, uint32_t accumulate) {
+#define MPSG_UMMA_A(hint)                                                            \
+  asm volatile(                                                                      \
+      "{\n\t.reg .pred p;\n\t"                                                       \
+      "setp.ne.b32 p, %4, 0;\n\t"                                                    \
+      "tcgen05.mma.cta_group::1.kind::f16.collector::a::" hint                       \
+      " [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),                                    \
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)                            \
+      : "memory")
+  if constexpr (OP == kFillA) MPSG_UMMA_A("fill");
+  else if constexpr (OP == kUseA) MPSG_UMMA_A("use");
+  else if constexpr (OP == kLastA) MPSG_UMMA_A("lastuse");
+  else umma_bf16(d_tmem, adesc, bdesc, idesc, accumulate);
+#undef MPSG_UMMA_A
+}
+
+// One lane of a converged warp. MMAs are issued behind it from code that the whole warp runs in step:
+// the compiler can then keep what the lanes agree on (descriptors, addresses) in uniform registers,
+// where tcgen05.mma wants its operands.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.b32 %0, 1, 0, p;\n\t}"
+      : "=r"(p));
+  return p != 0;
+}
+
+// A value that is the same in every lane of a converged warp, as a uniform register.
+__device__ __forceinline__ uint32_t warp_uniform(uint32_t x) {
+  return __reduce_max_sync(0xffffffffu, x);
+}
+
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile(
       "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(

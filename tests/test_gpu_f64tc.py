@@ -12,7 +12,8 @@ pytestmark = pytest.mark.gpu
 # orientations (few rows, few columns) and several blocks of different size in one launch
 SHAPES = [((33,), (33,), (33,)), ((128,), (64,), (32,)), ((129,), (65,), (257,)),
           ((40,), (513,), (256,)), ((600,), (41,), (255,)), ((1,), (200,), (40,)),
-          ((64, 7, 130), (257, 50, 40), (33, 1, 1031))]
+          ((64, 7, 130), (257, 50, 40), (33, 1, 1031)), ((81,), (80,), (1025,)),
+          ((40,), (33,), (8100,))]
 
 
 def pair(ms, ns, ks, seed=3):
@@ -32,7 +33,7 @@ def product(spaces, a, b, pipe=False):
         call("mpsg_contract_noalloc", A.ctx.handle, A.handle, i32arr((1, -1)), B.handle,
              i32arr((-1, 2)), C.handle)
     else:
-        C = mg.contract(A, (1, -1), B, (-1, 2), precision=0)
+        C = mg.matmul(A, B, precision=0)  # fused matrices: the tensor cores at every size
     f, out, p = C.to_flat(), [], 0
     for x, y in zip(a, b):
         n = x.shape[0] * y.shape[1]
@@ -44,14 +45,16 @@ def product(spaces, a, b, pipe=False):
 @pytest.mark.parametrize("ms,ns,ks", SHAPES)
 def test_rounded_once(ms, ns, ks):
     """Rounding the exact sum is at most 2^-53 of it; the digits left out add below 2^-57 of the
-    result's norm for normal data, so a quarter more covers both."""
+    result's norm for normal data, so a quarter more covers both. Beyond K = 8000 one more digit
+    group is summed in FP32: 2^-38 per drained sum of 64 columns against a result of 2^16."""
     spaces, a, b = pair(ms, ns, ks)
     rng = np.random.default_rng(1)
     for x, y, g in zip(a, b, product(spaces, a, b)):
         rows = np.sort(rng.choice(x.shape[0], min(x.shape[0], 24), replace=False))
         want = x[rows].astype(np.longdouble) @ y.astype(np.longdouble)
         err = np.linalg.norm((g[rows] - want).astype(float))
-        assert err <= 1.25 * 2.0 ** -53 * np.linalg.norm(want.astype(float))
+        tol = 1.25 * 2.0 ** -53 + (2.0 ** -52 if x.shape[1] > 8000 else 0.0)
+        assert err <= tol * np.linalg.norm(want.astype(float))
 
 
 @pytest.mark.parametrize("ms,ns,ks", SHAPES)
@@ -83,3 +86,56 @@ def test_values_outside_the_sliced_range():
         scale = np.abs(a).max(axis=1)[:, None] * np.abs(b).max(axis=0)[None, :]
     # K FMA roundings of at most 2^-53 of partial sums below K times the scale
     assert np.all(np.abs(g[rest] - h[rest]) <= 50 * 50 * 2.0 ** -53 * scale[rest])
+
+
+def noalloc(A, ia, B, ib, spaces):
+    C = mg.zeros(0, spaces)
+    call("mpsg_contract_noalloc", A.ctx.handle, A.handle, i32arr(ia), B.handle, i32arr(ib),
+         C.handle)
+    return C.to_flat()
+
+
+def test_special_values_read_in_place():
+    """The same through a contraction that reads its operands in place (A stored transposed, more
+    than the 2^21 FMAs that stay on the FP64 pipe)."""
+    (V, K, N), (a,), (b,) = pair((150,), (120,), (130,))
+    a[3, 4], a[12, 7], a[9, :], a[10], b[2, 8] = np.inf, np.nan, 0.0, a[10] * 1e-200, -np.inf
+    A = mg.from_flat(0, (mg.dual(K), V), a.T.ravel(order="F"))
+    B = mg.from_flat(0, (K, mg.dual(N)), b.ravel(order="F"))
+    g = mg.contract(A, (-1, 1), B, (-1, 2), precision=0).to_flat().reshape((150, 120), order="F")
+    h = noalloc(A, (-1, 1), B, (-1, 2), (V, mg.dual(N))).reshape((150, 120), order="F")
+    assert np.array_equal(np.isnan(g), np.isnan(h))
+    assert np.array_equal(g[[3, 10, 12]], h[[3, 10, 12]], equal_nan=True)
+    assert np.array_equal(g[:, 8], h[:, 8], equal_nan=True)
+    assert np.all(g[9, np.isfinite(h[9])] == 0.0)
+
+
+# thin kernel: every register variant (K up to 4, 8, 16, 32), both long axes, a unit's last rows
+@pytest.mark.parametrize("m,n,k", [(90001, 9, 3), (45003, 7, 8), (5, 60007, 9), (4001, 32, 31),
+                                   (31, 3300, 32)])
+def test_thin_kernel_same_fma_chain(m, n, k):
+    """Sparse thin operand with exact ones, zeros of both signs and non-finite values on either side:
+    skipped terms leave the FMA chain's bits as they are."""
+    (V, K, N), (a,), (b,) = pair((m,), (n,), (k,))
+    thin, long_ = (b, a) if m >= n else (a.T, b.T)
+    rng = np.random.default_rng(4)
+    thin[rng.random(thin.shape) < 0.5] = 0.0
+    thin[rng.random(thin.shape) < 0.2] = 1.0
+    thin[0, 0] = -0.0
+    long_[5, 0], long_[70, 1], long_[200, 2], long_[300, 0] = np.inf, np.nan, -0.0, -np.inf
+    A = mg.from_flat(0, (mg.dual(K), V), a.T.ravel(order="F"))
+    B = mg.from_flat(0, (K, mg.dual(N)), b.ravel(order="F"))
+    g = mg.contract(A, (-1, 1), B, (-1, 2), precision=0).to_flat()
+    h = noalloc(A, (-1, 1), B, (-1, 2), (V, mg.dual(N)))
+    assert np.array_equal(g, h, equal_nan=True)
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 1, 1), (33, 31, 40), (7, 200, 129), (64, 64, 64)])
+def test_small_kernel_same_fma_chain(m, n, k):
+    (V, K, N), (a,), (b,) = pair((m,), (n,), (k,))
+    a[0, 0] = np.inf if m > 1 else a[0, 0]
+    A = mg.from_flat(0, (mg.dual(K), V), a.T.ravel(order="F"))
+    B = mg.from_flat(0, (K, mg.dual(N)), b.ravel(order="F"))
+    g = mg.contract(A, (-1, 1), B, (-1, 2), precision=0).to_flat()
+    h = noalloc(A, (-1, 1), B, (-1, 2), (V, mg.dual(N)))
+    assert np.array_equal(g, h, equal_nan=True)
