@@ -396,6 +396,15 @@ struct Cfg {
 };
 constexpr int kExactThreads = 576;  // Cfg<S, BN>::kThreads (launch bound of the exact kernel)
 
+// MMA number `i` of `n` in a row that read the same A tile.
+__device__ __forceinline__ void umma_slices(int i, int n, uint32_t d, uint64_t ad, uint64_t bd,
+                                            uint32_t idesc, uint32_t acc) {
+  if (n == 1) umma_bf16(d, ad, bd, idesc, acc);
+  else if (i == 0) umma_bf16_a<kFillA>(d, ad, bd, idesc, acc);
+  else if (i == n - 1) umma_bf16_a<kLastA>(d, ad, bd, idesc, acc);
+  else umma_bf16_a<kUseA>(d, ad, bd, idesc, acc);
+}
+
 // 18 warps put 5 warps on one SM sub-partition (16K registers), which caps a thread at 96
 // registers; the epilogue drains TMEM in 16-column pieces to stay close to that
 template <int S, int BN>
@@ -471,64 +480,68 @@ __global__ void __launch_bounds__(kExactThreads, 1) split_gemm_kernel(
       }
     }
   } else if (warp == 1) {
-    // ---------------- MMA issuer ----------------
-    if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc(BM, CF::kBN);
-      int stage = 0;
-      uint32_t phase = 0;
-      int64_t use = 0;
-      bool issued = false;
-      for (int64_t i = 0; !*abort_flag; ++i) {
-        const int64_t pos = sched_pos(i, gridDim.x, blockIdx.x);
-        if (pos >= ntiles) break;
-        const int tw = tiles[pos].w;
-        const int nsteps = (int)((unsigned)tw >> 16) * CF::kPerRow;
-        for (int c0 = (tw & 0xffff) * CF::kPerRow; c0 < nsteps && !*abort_flag;
-             c0 += CF::kChunkSteps) {
-          const int buf = (int)(use % CF::kBufs);
-          const uint32_t bph = (uint32_t)((use / CF::kBufs) & 1);
-          if (!mbar_wait(&tempty[buf], bph ^ 1, abort_flag, err, 2)) break;
+    // ---------------- MMA issuer (the warp in step, one lane issues) ----------------
+    constexpr uint32_t idesc = make_idesc(BM, CF::kBN);
+    const uint32_t tmem = warp_uniform(tmem_base);
+    int stage = 0;
+    uint32_t phase = 0;
+    int64_t use = 0;
+    bool issued = false, ok = true;
+    for (int64_t i = 0; ok; ++i) {
+      const int64_t pos = sched_pos(i, gridDim.x, blockIdx.x);
+      if (pos >= ntiles) break;
+      const uint32_t tw = warp_uniform((uint32_t)tiles[pos].w);
+      const int nsteps = (int)(tw >> 16) * CF::kPerRow;
+      for (int c0 = (int)(tw & 0xffff) * CF::kPerRow; c0 < nsteps && ok; c0 += CF::kChunkSteps) {
+        const int buf = (int)(use % CF::kBufs);
+        const uint32_t bph = (uint32_t)((use / CF::kBufs) & 1);
+        ok = __all_sync(0xffffffffu, mbar_wait(&tempty[buf], bph ^ 1, abort_flag, err, 2));
+        if (!ok) break;
+        tc_fence_after();
+        const int c1 = min(nsteps, c0 + CF::kChunkSteps);
+        for (int ks = c0; ks < c1; ++ks) {
+          ok = __all_sync(0xffffffffu, mbar_wait(&full[stage], phase, abort_flag, err, 3));
+          if (!ok) break;
           tc_fence_after();
-          uint32_t init = 0;  // bit g: accumulator g already written in this chunk
-          const int c1 = min(nsteps, c0 + CF::kChunkSteps);
-          for (int ks = c0; ks < c1; ++ks) {
-            if (!mbar_wait(&full[stage], phase, abort_flag, err, 3)) break;
-            tc_fence_after();
-            const uint32_t sA = smem_u32(smem + stage * CF::kStageBytes);
-            const uint32_t sB = sA + S * CF::kABytes;
+          const uint32_t sA = warp_uniform(smem_u32(smem + stage * CF::kStageBytes));
+          const uint32_t sB = sA + S * CF::kABytes;
+          const uint32_t acc0 = ks == c0 ? 0u : 1u;  // a chunk's first products overwrite
+          issued = true;
+          if (elect_one()) {
 #pragma unroll
             for (int pa = 0; pa < S; ++pa) {
+              const uint64_t ad = CF::kBK == 64 ? sw128_desc(sA + pa * CF::kABytes)
+                                                : sw64_desc(sA + pa * CF::kABytes);
 #pragma unroll
-              for (int qb = 0; qb < S - pa; ++qb) {
-                const int g = pa + qb < CF::kAccs ? pa + qb : CF::kAccs - 1;  // accumulator
-                const uint32_t dcol = tmem_base + (uint32_t)((buf * CF::kAccs + g) * CF::kBN);
-                const uint64_t ad = CF::kBK == 64 ? sw128_desc(sA + pa * CF::kABytes)
-                                                  : sw64_desc(sA + pa * CF::kABytes);
-                const uint64_t bd = CF::kBK == 64 ? sw128_desc(sB + qb * CF::kBBytes)
-                                                  : sw64_desc(sB + qb * CF::kBBytes);
+              for (int kk = 0; kk < CF::kBK / 16; ++kk) {
 #pragma unroll
-                for (int kk = 0; kk < CF::kBK / 16; ++kk) {
-                  umma_bf16(dcol, ad + 2 * kk, bd + 2 * kk, idesc, (init >> g) & 1u);
-                  init |= 1u << g;
+                for (int qb = 0; qb < S - pa; ++qb) {
+                  const int g = pa + qb < CF::kAccs ? pa + qb : CF::kAccs - 1;  // accumulator
+                  const uint32_t d = tmem + (uint32_t)((buf * CF::kAccs + g) * CF::kBN);
+                  const uint64_t bd = CF::kBK == 64 ? sw128_desc(sB + qb * CF::kBBytes)
+                                                    : sw64_desc(sB + qb * CF::kBBytes);
+                  const uint32_t acc = pa == 0 && kk == 0 && qb < CF::kAccs ? acc0 : 1u;
+                  umma_slices(qb, S - pa, d, ad + 2 * kk, bd + 2 * kk, idesc, acc);
                 }
               }
             }
             umma_commit(&empty[stage]);
-            issued = true;
-            if (++stage == CF::kStages) {
-              stage = 0;
-              phase ^= 1;
-            }
+            if (ks == c1 - 1) umma_commit(&tfull[buf]);
           }
-          umma_commit(&tfull[buf]);
-          ++use;
+          __syncwarp();
+          if (++stage == CF::kStages) {
+            stage = 0;
+            phase ^= 1;
+          }
         }
+        ++use;
       }
-      if (issued) {  // make sure every MMA has retired before TMEM is released
-        umma_commit(drain);
-        volatile int no_abort = 0;
-        mbar_wait(drain, 0, &no_abort, err, 4);
-      }
+    }
+    if (issued) {  // make sure every MMA has retired before TMEM is released
+      if (elect_one()) umma_commit(drain);
+      __syncwarp();
+      volatile int no_abort = 0;
+      mbar_wait(drain, 0, &no_abort, err, 4);
     }
   } else {
     // ---------------- epilogue: warps 2..(2 + kEpiWarps - 1) ----------------
@@ -713,57 +726,61 @@ __global__ void __launch_bounds__(192, 1) split_gemm_fast_kernel(
       }
     }
   } else if (warp == 1) {
-    // ---------------- MMA issuer ----------------
-    if (lane == 0) {
-      constexpr uint32_t idesc = make_idesc(BM, BNF);
-      int stage = 0;
-      uint32_t phase = 0;
-      int64_t use = 0;
-      bool issued = false;
-      for (int64_t i = 0; !*abort_flag; ++i) {
-        const int64_t pos = sched_pos(i, gridDim.x, blockIdx.x);
-        if (pos >= ntiles) break;
-        const int nks = probs[tiles[pos].x].nks;
-        if (nks == 0) continue;
-        const int buf = (int)(use & 1);
-        const uint32_t bph = (uint32_t)((use >> 1) & 1);
-        if (!mbar_wait(&tempty[buf], bph ^ 1, abort_flag, err, 2)) break;
+    // ---------------- MMA issuer (the warp in step, one lane issues) ----------------
+    constexpr uint32_t idesc = make_idesc(BM, BNF);
+    const uint32_t tmem = warp_uniform(tmem_base);
+    int stage = 0;
+    uint32_t phase = 0;
+    int64_t use = 0;
+    bool issued = false, ok = true;
+    for (int64_t i = 0; ok; ++i) {
+      const int64_t pos = sched_pos(i, gridDim.x, blockIdx.x);
+      if (pos >= ntiles) break;
+      const int nks = (int)warp_uniform((uint32_t)probs[tiles[pos].x].nks);
+      if (nks == 0) continue;
+      const int buf = (int)(use & 1);
+      const uint32_t bph = (uint32_t)((use >> 1) & 1);
+      ok = __all_sync(0xffffffffu, mbar_wait(&tempty[buf], bph ^ 1, abort_flag, err, 2));
+      if (!ok) break;
+      tc_fence_after();
+      const uint32_t dcol = tmem + (uint32_t)(buf * BNF);
+      for (int kb = 0; kb < 2 * nks; ++kb) {
+        ok = __all_sync(0xffffffffu, mbar_wait(&full[stage], phase, abort_flag, err, 3));
+        if (!ok) break;
         tc_fence_after();
-        const uint32_t dcol = tmem_base + (uint32_t)(buf * BNF);
-        uint32_t acc = 0;
-        for (int kb = 0; kb < 2 * nks; ++kb) {
-          if (!mbar_wait(&full[stage], phase, abort_flag, err, 3)) break;
-          tc_fence_after();
-          const uint32_t sA = smem_u32(smem + stage * CF::kStageBytes);
-          const uint32_t sB = sA + S * CF::kABytes;
+        const uint32_t sA = warp_uniform(smem_u32(smem + stage * CF::kStageBytes));
+        const uint32_t sB = sA + S * CF::kABytes;
+        issued = true;
+        if (elect_one()) {
 #pragma unroll
           for (int pa = 0; pa < S; ++pa) {
+            const uint64_t ad = sw64_desc(sA + pa * CF::kABytes);
 #pragma unroll
-            for (int qb = 0; qb < S - pa; ++qb) {
-              const uint64_t ad = sw64_desc(sA + pa * CF::kABytes);
-              const uint64_t bd = sw64_desc(sB + qb * CF::kBBytes);
+            for (int kk = 0; kk < BKF / 16; ++kk) {
 #pragma unroll
-              for (int kk = 0; kk < BKF / 16; ++kk) {
-                umma_bf16(dcol, ad + 2 * kk, bd + 2 * kk, idesc, acc);
-                acc = 1;
+              for (int qb = 0; qb < S - pa; ++qb) {
+                const uint64_t bd = sw64_desc(sB + qb * CF::kBBytes);
+                const uint32_t acc = pa == 0 && kk == 0 && qb == 0 && kb == 0 ? 0u : 1u;
+                umma_slices(qb, S - pa, dcol, ad + 2 * kk, bd + 2 * kk, idesc, acc);
               }
             }
           }
           umma_commit(&empty[stage]);
-          issued = true;
-          if (++stage == CF::kStages) {
-            stage = 0;
-            phase ^= 1;
-          }
+          if (kb == 2 * nks - 1) umma_commit(&tfull[buf]);
         }
-        umma_commit(&tfull[buf]);
-        ++use;
+        __syncwarp();
+        if (++stage == CF::kStages) {
+          stage = 0;
+          phase ^= 1;
+        }
       }
-      if (issued) {
-        umma_commit(drain);
-        volatile int no_abort = 0;
-        mbar_wait(drain, 0, &no_abort, err, 4);
-      }
+      ++use;
+    }
+    if (issued) {
+      if (elect_one()) umma_commit(drain);
+      __syncwarp();
+      volatile int no_abort = 0;
+      mbar_wait(drain, 0, &no_abort, err, 4);
     }
   } else {
     // ---------------- epilogue: warps 2..5, one TMEM lane (= output row) per thread --------

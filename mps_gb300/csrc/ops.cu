@@ -228,6 +228,23 @@ DeviceTensor symmatrix(Context* ctx, const DeviceTensor& a, const std::vector<in
 // ------------------------------------------------------------------------------------------
 // block GEMM dispatch
 // ------------------------------------------------------------------------------------------
+// The arithmetic that a precision argument runs with: from 6 slices on the FP64 products of the
+// tensor cores (seven 9-bit slices, exact to the last bit of FP64), which are as many or fewer MMAs than
+// the 6- and 7-slice split products (1e-12 and 1e-14).
+static int arithmetic(int precision) {
+  if (precision == 0 || (precision >= 2 && precision < kFp64Slices)) return precision;
+  if (precision >= kFp64Slices && precision <= split::kMaxSlices) return 0;
+  throw Error(kErrUnsupported, "precision must be 0 (FP64) or 2..7 bf16 slices");
+}
+
+// Fewer slices pay only where MMAs are what takes the time. A split contraction fuses and packs its
+// operands and pads the MPO steps to whole tiles, none of which the FP64 contraction in place does: a
+// left environment update in us, FP64 / 4 / 5 slices: chi = 96 35 / 225 / 236, chi = 1024 140 / 596 /
+// 661, chi = 2048 327 / 1448 / 1684. So up to this many flops in the sector GEMMs that are not thin (a
+// few times the largest contraction of those updates, where 5 slices would save 0.3 ms of MMAs)
+// a contraction asked for with slices gets FP64 results.
+constexpr double kSplitContractFlops = 2e10;
+
 static void run_gemm(Context* ctx, DevGemmPlan& g, const double* A, const double* B,
                      double* C, int precision) {
   if (precision == 0) {
@@ -248,6 +265,7 @@ static void run_gemm(Context* ctx, DevGemmPlan& g, const double* A, const double
 }
 
 DeviceTensor matmul(Context* ctx, const DeviceTensor& a, const DeviceTensor& b, int precision) {
+  precision = arithmetic(precision);
   std::string key = "G|" + meta_key(a.meta) + "*" + meta_key(b.meta);
   std::shared_ptr<DevGemmPlan> g;
   std::shared_ptr<TensorMeta> outmeta;
@@ -350,10 +368,14 @@ DeviceTensor contract(Context* ctx, const DeviceTensor& a, const std::vector<int
     if (scalar) *scalar = s;
     return DeviceTensor();
   }
+  precision = arithmetic(precision);
   DeviceTensor t;
   t.ctx = ctx;
   t.meta = p->host->split.out;
-  if (DirectPlan* d = precision == 0 ? direct_plan(ctx, *p) : nullptr) {
+  DirectPlan* d = precision == 0 || p->host->tiled_flops() <= kSplitContractFlops
+                      ? direct_plan(ctx, *p)
+                      : nullptr;
+  if (d) {
     t.buf = alloc_buffer(ctx, t.meta.total);
     if (launch_direct(ctx, *d, a.data(), b.data(), t.data())) return t;
     t.buf.reset();
@@ -379,7 +401,8 @@ static const std::vector<int> kH4A = {1, 2, 3, -1, -2}, kH4B = {-2, -1, 4};
 DeviceTensor applymps2site(Context* ctx, const DeviceTensor& v, const DeviceTensor& envL,
                            const DeviceTensor& envR, const DeviceTensor& W1,
                            const DeviceTensor& W2, int precision) {
-  if (precision != 0) {  // tensor-core path: prepared (W-folded) operator, built per call here
+  precision = arithmetic(precision);
+  if (precision != 0) {  // split-precision path: prepared (W-folded) operator, built per call here
     auto op = heff_create(ctx, v.meta, envL, envR, W1, W2, precision);
     return heff_apply(*op, v);
   }
@@ -447,7 +470,7 @@ DeviceTensor applymps2site_host(Context* ctx, const DeviceTensor& v, const Devic
   }
   MPSG_CUDA(cudaEventRecord(ctx->copy_ev[2], cs));  // v
   DeviceTensor out;
-  if (precision != 0) {
+  if (arithmetic(precision) != 0) {
     auto op = heff_create(ctx, v.meta, envL, envR, W1, W2, precision, ctx->copy_ev[0],
                           ctx->copy_ev[1]);
     MPSG_CUDA(cudaStreamWaitEvent(ctx->stream, ctx->copy_ev[2], 0));
@@ -642,14 +665,16 @@ std::shared_ptr<HeffOp> heff_create(Context* ctx, const TensorMeta& vmeta, const
                                     cudaEvent_t wait_right) {
   auto op = std::make_shared<HeffOp>();
   op->ctx = ctx;
-  op->precision = precision;
   op->vmeta = vmeta;
   op->ref_flops = applymps2site_flops(ctx, vmeta, envL.meta, envR.meta, W1.meta, W2.meta);
-  if (precision == 0) {
-    op->envL = envL;
-    op->envR = envR;
-    op->W1 = W1;
-    op->W2 = W2;
+  op->precision = arithmetic(precision);
+  if (op->precision == 0) {
+    // precision 0 reads the tensors at every application; a slice count takes them as they are now
+    const bool keep = precision != 0;
+    op->envL = keep ? copy_tensor(ctx, envL) : envL;
+    op->envR = keep ? copy_tensor(ctx, envR) : envR;
+    op->W1 = keep ? copy_tensor(ctx, W1) : W1;
+    op->W2 = keep ? copy_tensor(ctx, W2) : W2;
     return op;
   }
   HeffParts H = heff_parts(ctx, vmeta, envL, envR, W1, W2, precision);

@@ -6,6 +6,10 @@
 
 namespace mpsg {
 
+// Slice counts from this one on run as FP64 (see arithmetic() in ops.cu); batched operators keep their
+// split-precision slices.
+constexpr int kFp64Slices = 6;
+
 void context_init(Context* ctx, int device);
 
 DeviceTensor new_tensor(Context* ctx, const TensorMeta& meta, bool zero);

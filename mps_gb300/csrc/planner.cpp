@@ -761,6 +761,13 @@ std::shared_ptr<ContractPlan> plan_contract(const TensorMeta& A, const std::vect
   return P;
 }
 
+double ContractPlan::tiled_flops() const {
+  double f = 0;
+  for (const GemmTask& g : mm.gemms)
+    if (g.K > 32 || (g.M > 32 && g.N > 32)) f += 2.0 * g.M * g.N * g.K;
+  return f;
+}
+
 static void apply_tasks_host(const std::vector<CopyTask>& tasks, const std::vector<int64_t>& src,
                              std::vector<int64_t>& dst) {
   for (const CopyTask& t : tasks) {

@@ -177,6 +177,7 @@ struct ContractPlan {
   RelegPlan split;
   bool scalar = false;  // every leg contracted: result is a number
   double flops = 0;
+  double tiled_flops() const;  // of the sector GEMMs with K, or both M and N, above 32
   // arguments of the pieces, kept to compose plans of chained contractions
   std::vector<int> rowsA, colsA, rowsB, colsB;  // SymMatrix index lists (1-based)
   std::vector<Space> rlegs, clegs;              // legs of the split
