@@ -1,7 +1,6 @@
 // Tensor-level operations: plan lookup (cached per structure), scratch management and the
 // launch sequences of each SymTensors operation.
 #include <algorithm>
-#include <sstream>
 
 #include "direct.hpp"
 #include "ops.hpp"
@@ -156,12 +155,6 @@ void require_similar(const DeviceTensor& a, const DeviceTensor& b, const char* m
 // ------------------------------------------------------------------------------------------
 // releg
 // ------------------------------------------------------------------------------------------
-static std::string vkey(const std::vector<int>& v) {
-  std::ostringstream os;
-  for (int x : v) os << x << ',';
-  return os.str();
-}
-
 static std::string spaces_key(const std::vector<Space>& sp) {
   TensorMeta m;
   m.space = sp;
@@ -193,7 +186,7 @@ static DeviceTensor run_releg(Context* ctx, const DevReleg& p, const DeviceTenso
 }
 
 DeviceTensor permutelegs(Context* ctx, const DeviceTensor& a, const std::vector<int>& perm1) {
-  auto p = releg_plan(ctx, "P|" + meta_key(a.meta) + vkey(perm1),
+  auto p = releg_plan(ctx, "P|" + meta_key(a.meta) + index_key(perm1),
                       [&] { return plan_permutelegs(a.meta, perm1); });
   DeviceTensor t = run_releg(ctx, *p, a);
   t.diag = a.diag;
@@ -201,20 +194,20 @@ DeviceTensor permutelegs(Context* ctx, const DeviceTensor& a, const std::vector<
 }
 
 DeviceTensor fuselegs(Context* ctx, const DeviceTensor& a, int l1, int n, bool dual) {
-  auto p = releg_plan(ctx, "F|" + meta_key(a.meta) + vkey({l1, n, (int)dual}),
+  auto p = releg_plan(ctx, "F|" + meta_key(a.meta) + index_key({l1, n, (int)dual}),
                       [&] { return plan_fuselegs(a.meta, l1, n, dual); });
   return run_releg(ctx, *p, a);
 }
 
 DeviceTensor splitleg(Context* ctx, const DeviceTensor& a, int l1, const std::vector<Space>& sp) {
-  auto p = releg_plan(ctx, "S|" + meta_key(a.meta) + vkey({l1}) + spaces_key(sp),
+  auto p = releg_plan(ctx, "S|" + meta_key(a.meta) + index_key({l1}) + spaces_key(sp),
                       [&] { return plan_splitleg(a.meta, l1, sp); });
   return run_releg(ctx, *p, a);
 }
 
 DeviceTensor symmatrix(Context* ctx, const DeviceTensor& a, const std::vector<int>& rows,
                        const std::vector<int>& cols) {
-  auto p = releg_plan(ctx, "M|" + meta_key(a.meta) + vkey(rows) + "/" + vkey(cols), [&] {
+  auto p = releg_plan(ctx, "M|" + meta_key(a.meta) + index_key(rows) + "/" + index_key(cols), [&] {
     FusePlan f = plan_symmatrix(a.meta, rows, cols);
     RelegPlan r;
     r.out = f.out;
@@ -291,7 +284,7 @@ std::shared_ptr<DevContract> get_contract_plan(Context* ctx, const TensorMeta& A
                                                const std::vector<int>& idxA,
                                                const TensorMeta& B,
                                                const std::vector<int>& idxB) {
-  std::string key = "C|" + meta_key(A) + vkey(idxA) + "|" + meta_key(B) + vkey(idxB);
+  std::string key = "C|" + meta_key(A) + index_key(idxA) + "|" + meta_key(B) + index_key(idxB);
   if (auto hit = ctx->contract_cache.get(key)) return hit;
   auto p = std::make_shared<DevContract>();
   p->host = plan_contract(A, idxA, B, idxB);

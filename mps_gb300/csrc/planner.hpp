@@ -192,8 +192,10 @@ void check_composition(const std::vector<CopyTask>& step1, int64_t n_src, int64_
 std::shared_ptr<ContractPlan> plan_contract(const TensorMeta& A, const std::vector<int>& idxA,
                                             const TensorMeta& B, const std::vector<int>& idxB);
 
-// Serialised key of a tensor's structure (charge + spaces), used by the plan cache.
+// Serialised keys of a tensor's structure (charge + spaces) and of an index list, used by the plan
+// caches (bytes, self-delimiting).
 std::string meta_key(const TensorMeta& m);
+std::string index_key(const std::vector<int>& v);
 
 // Host self-checks of task lists (run by tests before anything reaches a GPU): every source and
 // destination address in range, every destination element written exactly once, every GEMM
