@@ -21,8 +21,9 @@ CSRC = os.path.join(HERE, "csrc")
 BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libmpsgb300.so")
 
-SOURCES = ["planner.cpp", "contract_map.cpp", "ops.cu", "capi.cu", "kernels_copy.cu", "kernels_f64.cu", "linalg.cu",
-           "krylov.cu", "kernels_split.cu", "kernels_f64tc.cu", "kernels_map.cu", "noalloc.cu", "batch.cu"]
+SOURCES = ["planner.cpp", "contract_map.cpp", "ops.cu", "capi.cu", "kernels_copy.cu",
+           "kernels_f64.cu", "kernels_f64tc.cu", "kernels_map.cu", "kernels_split.cu", "linalg.cu",
+           "svd_small.cu", "krylov.cu", "noalloc.cu", "batch.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 CFLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-Wall",
           "--expt-relaxed-constexpr", "-I", CSRC]

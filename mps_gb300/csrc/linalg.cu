@@ -8,11 +8,13 @@
 #include <algorithm>
 #include <cstdlib>
 #include <cmath>
+#include <cstring>
 #include <exception>
 #include <functional>
 #include <thread>
 
 #include "linalg.hpp"
+#include "svd_small.hpp"
 
 namespace mpsg {
 
@@ -88,6 +90,28 @@ __global__ void set_diag_kernel(double* __restrict__ dst, const double* __restri
     dst[i + k * i] = s[i];
 }
 
+// One kept block of an SVD's outputs: u <- U[:, :r], s <- diag(S[:r]) on a zeroed block, v <- V[:, :r]^T.
+struct OutBlock {
+  const double *U, *S, *V;
+  double *u, *s, *v;
+  int64_t M, N, r;
+};
+
+__global__ void __launch_bounds__(256) svd_outputs_kernel(const OutBlock* __restrict__ blocks) {
+  const OutBlock B = blocks[blockIdx.y];
+  const int64_t nu = B.M * B.r, nv = B.N * B.r;
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < nu + nv;
+       e += (int64_t)gridDim.x * blockDim.x) {
+    if (e < nu) {
+      B.u[e] = B.U[e];
+      if (e < B.r) B.s[e + B.r * e] = B.S[e];
+    } else {  // consecutive threads write one column of v
+      const int64_t f = e - nu, j = f / B.r, i = f - j * B.r;
+      B.v[f] = B.V[j + B.N * i];
+    }
+  }
+}
+
 // dst (r x n, column-major) = first r columns of src (n x k, column-major) transposed
 __global__ void transpose_prefix_kernel(double* __restrict__ dst, const double* __restrict__ src,
                                         int64_t r, int64_t n) {
@@ -158,7 +182,8 @@ unsigned grid_for(int64_t n) { return (unsigned)std::min<int64_t>((n + 255) / 25
 // list is issued by its own host thread: cuSOLVER's eigen- and SVD solvers block the calling
 // thread on large blocks, which would otherwise serialise the lanes.
 void run_on_lanes(Context* ctx, SolverLanes& L, size_t nb, const std::function<double(size_t)>& cost,
-                  const std::function<void(int, size_t)>& work) {
+                  const std::function<void(int, size_t)>& work,
+                  const std::function<void()>& meanwhile = nullptr) {
   std::vector<size_t> order(nb);
   for (size_t b = 0; b < nb; ++b) order[b] = b;
   std::stable_sort(order.begin(), order.end(),
@@ -188,6 +213,12 @@ void run_on_lanes(Context* ctx, SolverLanes& L, size_t nb, const std::function<d
   std::vector<std::thread> threads;
   for (int i = 1; i < kLanes; ++i)
     if (!list[i].empty()) threads.emplace_back(run_lane, i);
+  std::exception_ptr aside;
+  try {
+    if (meanwhile) meanwhile();
+  } catch (...) {
+    aside = std::current_exception();
+  }
   run_lane(0);
   for (auto& t : threads) t.join();
   for (int i = 0; i < kLanes; ++i) {
@@ -197,6 +228,7 @@ void run_on_lanes(Context* ctx, SolverLanes& L, size_t nb, const std::function<d
   }
   for (int i = 0; i < kLanes; ++i)
     if (failure[i]) std::rethrow_exception(failure[i]);
+  if (aside) std::rethrow_exception(aside);
 }
 
 // Complex block assembled from its real and imaginary planes (rows x cols, column-major):
@@ -229,7 +261,9 @@ __global__ void cplx_extract_kernel(double* __restrict__ dre, double* __restrict
 struct BlockSVD {
   int c1, c2;
   int64_t M, N, k;
-  std::shared_ptr<Buffer> U, S, V;  // U: M x k, S: k, V: N x k (all column-major)
+  double *U = nullptr, *S = nullptr, *V = nullptr;  // U: M x k, S: k, V: N x k (column-major)
+  int64_t offS = 0;                          // of S among the call's singular values
+  std::shared_ptr<Buffer> uv;                // U and V, unless they are part of a larger buffer
   std::shared_ptr<Buffer> work, aux, wbuf;  // temporaries, kept until the lanes are joined
   std::shared_ptr<Buffer> ref;              // second-level Gram workspace (density matrix)
   int lwork = 0;
@@ -254,9 +288,9 @@ double refine_threshold() {  // MPSG_GRAM_REFINE overrides it (0: no second leve
 // on the context stream; this only enqueues work on the lane's stream.
 void prepare_exact(Context* ctx, cusolverDnHandle_t h, BlockSVD& B) {
   const int64_t M = B.M, N = B.N, k = B.k;
-  B.U = alloc_buffer(ctx, M * k);
-  B.S = alloc_buffer(ctx, k);
-  B.V = alloc_buffer(ctx, N * k);
+  B.uv = alloc_buffer(ctx, (M + N) * k);
+  B.U = B.uv->ptr;
+  B.V = B.U + M * k;
   B.work = alloc_buffer(ctx, M * N);
   B.aux = alloc_buffer(ctx, k * k);
   const int64_t m = std::max(M, N), n = std::min(M, N);
@@ -271,20 +305,20 @@ void run_exact(Context* ctx, cudaStream_t st, cusolverDnHandle_t h, const double
     MPSG_CUDA(cudaMemcpyAsync(B.work->ptr, A, sizeof(double) * M * N, cudaMemcpyDeviceToDevice,
                               st));
     // A = U S VT with VT (N x N) in aux; V = VT^T
-    MPSG_SOLVER(cusolverDnDgesvd(h, 'S', 'S', (int)M, (int)N, B.work->ptr, (int)M, B.S->ptr,
-                                 B.U->ptr, (int)M, B.aux->ptr, (int)N, B.wbuf->ptr, B.lwork,
+    MPSG_SOLVER(cusolverDnDgesvd(h, 'S', 'S', (int)M, (int)N, B.work->ptr, (int)M, B.S,
+                                 B.U, (int)M, B.aux->ptr, (int)N, B.wbuf->ptr, B.lwork,
                                  nullptr, dinfo));
     dim3 g((unsigned)((N + 31) / 32), (unsigned)((N + 31) / 32));
-    transpose_prefix_kernel<<<g, dim3(32, 8), 0, st>>>(B.V->ptr, B.aux->ptr, N, N);
+    transpose_prefix_kernel<<<g, dim3(32, 8), 0, st>>>(B.V, B.aux->ptr, N, N);
   } else {
     // A^T (N x M) = U' S V'^T  =>  A = V' S U'^T: V = U' (N x M), U = V'^T^T from aux (M x M)
     dim3 g((unsigned)((N + 31) / 32), (unsigned)((M + 31) / 32));
     transpose_prefix_kernel<<<g, dim3(32, 8), 0, st>>>(B.work->ptr, A, N, M);
-    MPSG_SOLVER(cusolverDnDgesvd(h, 'S', 'S', (int)N, (int)M, B.work->ptr, (int)N, B.S->ptr,
-                                 B.V->ptr, (int)N, B.aux->ptr, (int)M, B.wbuf->ptr, B.lwork,
+    MPSG_SOLVER(cusolverDnDgesvd(h, 'S', 'S', (int)N, (int)M, B.work->ptr, (int)N, B.S,
+                                 B.V, (int)N, B.aux->ptr, (int)M, B.wbuf->ptr, B.lwork,
                                  nullptr, dinfo));
     dim3 g2((unsigned)((M + 31) / 32), (unsigned)((M + 31) / 32));
-    transpose_prefix_kernel<<<g2, dim3(32, 8), 0, st>>>(B.U->ptr, B.aux->ptr, M, M);
+    transpose_prefix_kernel<<<g2, dim3(32, 8), 0, st>>>(B.U, B.aux->ptr, M, M);
   }
   MPSG_CUDA(cudaGetLastError());
   (void)k;
@@ -305,14 +339,14 @@ void run_jacobi(Context* ctx, const double* A, BlockSVD& B) {
   MPSG_SOLVER(cusolverDnCreateGesvdjInfo(&params));
   int lwork = 0;
   MPSG_SOLVER(cusolverDnDgesvdj_bufferSize(h, CUSOLVER_EIG_MODE_VECTOR, 1, (int)M, (int)N,
-                                           work->ptr, (int)M, B.S->ptr, B.U->ptr, (int)M,
-                                           B.V->ptr, (int)N, &lwork, params));
+                                           work->ptr, (int)M, B.S, B.U, (int)M,
+                                           B.V, (int)N, &lwork, params));
   auto wbuf = alloc_buffer(ctx, std::max(lwork, 1));
   int* dinfo = nullptr;
   MPSG_CUDA(cudaMallocAsync((void**)&dinfo, sizeof(int), ctx->stream));
   MPSG_CUDA(cudaStreamSynchronize(ctx->stream));
   MPSG_SOLVER(cusolverDnDgesvdj(h, CUSOLVER_EIG_MODE_VECTOR, 1, (int)M, (int)N, work->ptr,
-                                (int)M, B.S->ptr, B.U->ptr, (int)M, B.V->ptr, (int)N, wbuf->ptr,
+                                (int)M, B.S, B.U, (int)M, B.V, (int)N, wbuf->ptr,
                                 lwork, dinfo, params));
   int info = 0;
   MPSG_CUDA(cudaMemcpyAsync(&info, dinfo, sizeof(int), cudaMemcpyDeviceToHost, st));
@@ -330,9 +364,9 @@ void run_jacobi(Context* ctx, const double* A, BlockSVD& B) {
 // projection of A on the kept singular subspace, which is all a sweep uses of it.
 void prepare_gram(Context* ctx, cusolverDnHandle_t h, BlockSVD& B, bool left) {
   const int64_t M = B.M, N = B.N, k = B.k, n = left ? M : N;
-  B.U = alloc_buffer(ctx, M * k);
-  B.S = alloc_buffer(ctx, k);
-  B.V = alloc_buffer(ctx, N * k);
+  B.uv = alloc_buffer(ctx, (M + N) * k);
+  B.U = B.uv->ptr;
+  B.V = B.U + M * k;
   B.work = alloc_buffer(ctx, n * n);
   B.aux = alloc_buffer(ctx, n);
   MPSG_SOLVER(cusolverDnDsyevd_bufferSize(h, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_LOWER,
@@ -359,9 +393,9 @@ void run_gram(Context* ctx, cudaStream_t st, cusolverDnHandle_t h, cublasHandle_
                           (int)M, &zero, G, (int)N));
   MPSG_SOLVER(cusolverDnDsyevd(h, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_LOWER, (int)n, G,
                                (int)n, B.aux->ptr, B.wbuf->ptr, B.lwork, dinfo));
-  double* X = left ? B.U->ptr : B.V->ptr;  // orthonormal factor
-  double* Y = left ? B.V->ptr : B.U->ptr;  // the other one
-  top_eigpairs_kernel<<<grid_for(n * k), 256, 0, st>>>(X, B.S->ptr, G, B.aux->ptr, n, k);
+  double* X = left ? B.U : B.V;  // orthonormal factor
+  double* Y = left ? B.V : B.U;  // the other one
+  top_eigpairs_kernel<<<grid_for(n * k), 256, 0, st>>>(X, B.S, G, B.aux->ptr, n, k);
   const int64_t rows = left ? N : M;
   // second level: the eigenvalues decide how many trailing columns of X to redo
   std::vector<double> w(n);
@@ -403,10 +437,10 @@ void run_gram(Context* ctx, cudaStream_t st, cusolverDnHandle_t h, cublasHandle_
   else  // U (M x k) = A V
     MPSG_BLAS(cublasDgemm(bl, CUBLAS_OP_N, CUBLAS_OP_N, (int)M, (int)k, (int)N, &one, A, (int)M,
                           X, (int)N, &zero, Y, (int)M));
-  col_norms_kernel<<<(unsigned)std::min<int64_t>((k + 7) / 8, 1184), 256, 0, st>>>(Y, B.S->ptr,
+  col_norms_kernel<<<(unsigned)std::min<int64_t>((k + 7) / 8, 1184), 256, 0, st>>>(Y, B.S,
                                                                                  rows, k);
-  running_min_kernel<<<1, 1, 0, st>>>(B.S->ptr, k);
-  scale_cols_inv_kernel<<<grid_for(rows * k), 256, 0, st>>>(Y, B.S->ptr, rows, k);
+  running_min_kernel<<<1, 1, 0, st>>>(B.S, k);
+  scale_cols_inv_kernel<<<grid_for(rows * k), 256, 0, st>>>(Y, B.S, rows, k);
   MPSG_CUDA(cudaGetLastError());
 }
 
@@ -466,10 +500,11 @@ SVDResult svd_blocks(Context* ctx, const DeviceTensor& A, bool truncate, int64_t
   if (method != kSvdExact && method != kSvdGramLeft && method != kSvdGramRight)
     throw Error(kErrArgument, "unknown SVD method");
   const size_t nb = A.meta.nblocks();
-  SolverLanes& L = lanes(ctx);
   std::vector<BlockSVD> blocks(nb);
   std::vector<std::vector<double>> S(nb);
-  // all buffers first (stream-ordered on the context stream), then fork the lanes
+  // one allocation for the singular values and states of all blocks, read back in one copy
+  int64_t nS = 0;
+  std::vector<size_t> small, large;
   for (size_t b = 0; b < nb; ++b) {
     BlockSVD& B = blocks[b];
     B.c1 = A.meta.sec.labels(b)[0];
@@ -477,71 +512,96 @@ SVDResult svd_blocks(Context* ctx, const DeviceTensor& A, bool truncate, int64_t
     B.M = A.meta.sec.sizes(b)[0];
     B.N = A.meta.sec.sizes(b)[1];
     B.k = std::min(B.M, B.N);
-    if (method == kSvdExact) prepare_exact(ctx, L.sol[0], B);
-    else prepare_gram(ctx, L.sol[0], B, method == kSvdGramLeft);
+    B.offS = nS;
+    nS += B.k;
+    (small_svd_fits(B.M, B.N) ? small : large).push_back(b);
   }
-  int* dinfo = nullptr;
-  if (nb) {
-    MPSG_CUDA(cudaMallocAsync((void**)&dinfo, sizeof(int) * nb, ctx->stream));
-    MPSG_CUDA(cudaMemsetAsync(dinfo, 0, sizeof(int) * nb, ctx->stream));
+  auto values = alloc_buffer(ctx, nS + (int64_t)(nb + 1) / 2);
+  int* dinfo = (int*)(values->ptr + nS);
+  if (nb) MPSG_CUDA(cudaMemsetAsync(dinfo, 0, sizeof(int) * nb, ctx->stream));
+  for (BlockSVD& B : blocks) B.S = values->ptr + B.offS;
+  // small blocks: Jacobi in one launch, whatever the method (it satisfies the density-matrix ones
+  // too: both factors orthonormal, u s v = A)
+  int64_t nf = 0;
+  for (size_t b : small) nf += (blocks[b].M + blocks[b].N) * blocks[b].k;
+  auto factors = alloc_buffer(ctx, nf);
+  std::vector<SmallSvdBlock> js;
+  nf = 0;
+  for (size_t b : small) {
+    BlockSVD& B = blocks[b];
+    B.U = factors->ptr + nf;
+    B.V = B.U + B.M * B.k;
+    nf += (B.M + B.N) * B.k;
+    js.push_back(SmallSvdBlock{A.data() + A.meta.off[b], B.U, B.S, B.V, dinfo + b, (int32_t)B.M,
+                               (int32_t)B.N});
   }
-  auto cost = [&](size_t b) {
-    const double m = (double)std::max(blocks[b].M, blocks[b].N);
-    const double n = (double)blocks[b].k;
-    return m * n * n + n * n * n;
-  };
-  run_on_lanes(ctx, L, nb, cost, [&](int lane, size_t b) {
-    const double* Ab = A.data() + A.meta.off[b];
-    if (method == kSvdExact) run_exact(ctx, L.st[lane], L.sol[lane], Ab, blocks[b], dinfo + b);
-    else run_gram(ctx, L.st[lane], L.sol[lane], L.blas[lane], Ab, blocks[b],
-                  method == kSvdGramLeft, dinfo + b);
-  });
-  ctx->kernel_launches += (int64_t)nb * (method == kSvdExact ? 1 : 4);
   std::vector<int> info(nb, 0);
-  if (nb)
-    MPSG_CUDA(cudaMemcpyAsync(info.data(), dinfo, sizeof(int) * nb, cudaMemcpyDeviceToHost,
-                              ctx->stream));
-  for (size_t b = 0; b < nb; ++b) {
-    S[b].resize(blocks[b].k);
-    MPSG_CUDA(cudaMemcpyAsync(S[b].data(), blocks[b].S->ptr, sizeof(double) * blocks[b].k,
+  auto factorise = [&](const std::vector<size_t>& list, const std::function<void()>& meanwhile) {
+    if (list.empty()) {
+      meanwhile();
+    } else {
+      SolverLanes& L = lanes(ctx);
+      // all buffers first (stream-ordered on the context stream), then fork the lanes
+      for (size_t b : list) {
+        if (method == kSvdExact) prepare_exact(ctx, L.sol[0], blocks[b]);
+        else prepare_gram(ctx, L.sol[0], blocks[b], method == kSvdGramLeft);
+      }
+      auto cost = [&](size_t i) {
+        const BlockSVD& B = blocks[list[i]];
+        const double m = (double)std::max(B.M, B.N), n = (double)B.k;
+        return m * n * n + n * n * n;
+      };
+      run_on_lanes(ctx, L, list.size(), cost, [&](int lane, size_t i) {
+        const size_t b = list[i];
+        const double* Ab = A.data() + A.meta.off[b];
+        if (method == kSvdExact) run_exact(ctx, L.st[lane], L.sol[lane], Ab, blocks[b], dinfo + b);
+        else run_gram(ctx, L.st[lane], L.sol[lane], L.blas[lane], Ab, blocks[b],
+                      method == kSvdGramLeft, dinfo + b);
+      }, meanwhile);
+      ctx->kernel_launches += (int64_t)list.size() * (method == kSvdExact ? 1 : 4);
+    }
+    std::vector<double> host(nS + (nb + 1) / 2);
+    MPSG_CUDA(cudaMemcpyAsync(host.data(), values->ptr, sizeof(double) * host.size(),
                               cudaMemcpyDeviceToHost, ctx->stream));
+    MPSG_CUDA(cudaStreamSynchronize(ctx->stream));
+    std::memcpy(info.data(), host.data() + nS, sizeof(int) * nb);
+    for (size_t b = 0; b < nb; ++b)
+      S[b].assign(host.begin() + blocks[b].offS, host.begin() + blocks[b].offS + blocks[b].k);
+  };
+  if (nb) factorise(large, [&] { launch_small_svd(ctx, js); });
+  std::vector<size_t> refused;  // left to the solvers by the small-block kernel
+  for (size_t b : small)
+    if (info[b]) refused.push_back(b);
+  if (!refused.empty()) {
+    MPSG_CUDA(cudaMemsetAsync(dinfo, 0, sizeof(int) * nb, ctx->stream));
+    std::vector<int> before(info);
+    factorise(refused, nullptr);
+    for (size_t b : large) info[b] = before[b];
   }
-  MPSG_CUDA(cudaStreamSynchronize(ctx->stream));
-  if (dinfo) cudaFreeAsync(dinfo, ctx->stream);
   for (size_t b = 0; b < nb; ++b) {
     if (info[b] == 0) continue;
+    BlockSVD& B = blocks[b];
+    int i1 = 1;
     if (method != kSvdExact) {
       // the Gram eigensolver failed on this block: factorise it exactly instead (QR-iteration
       // SVD, then Jacobi), which also leaves u and v orthonormal with u s v = A
-      BlockSVD E;
-      E.c1 = blocks[b].c1;
-      E.c2 = blocks[b].c2;
-      E.M = blocks[b].M;
-      E.N = blocks[b].N;
-      E.k = blocks[b].k;
-      prepare_exact(ctx, L.sol[0], E);
+      SolverLanes& L = lanes(ctx);
+      prepare_exact(ctx, L.sol[0], B);
       int* d1 = nullptr;
       MPSG_CUDA(cudaMallocAsync((void**)&d1, sizeof(int), ctx->stream));
       MPSG_CUDA(cudaMemsetAsync(d1, 0, sizeof(int), ctx->stream));
       MPSG_CUDA(cudaEventRecord(L.fork, ctx->stream));
       MPSG_CUDA(cudaStreamWaitEvent(L.st[0], L.fork, 0));
-      run_exact(ctx, L.st[0], L.sol[0], A.data() + A.meta.off[b], E, d1);
+      run_exact(ctx, L.st[0], L.sol[0], A.data() + A.meta.off[b], B, d1);
       ctx->kernel_launches += 1;
       MPSG_CUDA(cudaEventRecord(L.join[0], L.st[0]));
       MPSG_CUDA(cudaStreamWaitEvent(ctx->stream, L.join[0], 0));
-      int i1 = 0;
       MPSG_CUDA(cudaMemcpyAsync(&i1, d1, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream));
       MPSG_CUDA(cudaStreamSynchronize(ctx->stream));
       cudaFreeAsync(d1, ctx->stream);
-      if (i1 != 0) run_jacobi(ctx, A.data() + A.meta.off[b], E);
-      blocks[b].U = E.U;
-      blocks[b].S = E.S;
-      blocks[b].V = E.V;
-    } else {
-      run_jacobi(ctx, A.data() + A.meta.off[b], blocks[b]);
     }
-    MPSG_CUDA(cudaMemcpy(S[b].data(), blocks[b].S->ptr, sizeof(double) * blocks[b].k,
-                         cudaMemcpyDeviceToHost));
+    if (i1 != 0) run_jacobi(ctx, A.data() + A.meta.off[b], B);
+    MPSG_CUDA(cudaMemcpy(S[b].data(), B.S, sizeof(double) * B.k, cudaMemcpyDeviceToHost));
   }
   std::vector<int64_t> ns(nb);
   int64_t total = 0;
@@ -573,6 +633,7 @@ SVDResult svd_blocks(Context* ctx, const DeviceTensor& A, bool truncate, int64_t
   R.s = new_tensor(ctx, ms, true);
   R.s.diag = true;
   R.v = new_tensor(ctx, mv, false);
+  std::vector<OutBlock> ob;
   for (size_t b = 0; b < nb; ++b) {
     const int64_t r = ns[b];
     if (r <= 0) continue;
@@ -580,16 +641,19 @@ SVDResult svd_blocks(Context* ctx, const DeviceTensor& A, bool truncate, int64_t
     int su[2] = {B.c1, B.c1}, ss[2] = {B.c1, B.c2}, sv[2] = {B.c2, B.c2};
     long iu = mu.find(su), is = ms.find(ss), iv = mv.find(sv);
     if (iu < 0 || is < 0 || iv < 0) throw Error(kErrSpaceMismatch, "svd: output sector missing");
-    // U[:, 1:r] is the contiguous prefix of the column-major U
-    MPSG_CUDA(cudaMemcpyAsync(R.u.data() + mu.off[iu], B.U->ptr, sizeof(double) * B.M * r,
-                              cudaMemcpyDeviceToDevice, ctx->stream));
-    set_diag_kernel<<<1, 256, 0, ctx->stream>>>(R.s.data() + ms.off[is], B.S->ptr, r);
-    dim3 g((unsigned)((r + 31) / 32), (unsigned)((B.N + 31) / 32));
-    transpose_prefix_kernel<<<g, dim3(32, 8), 0, ctx->stream>>>(R.v.data() + mv.off[iv],
-                                                               B.V->ptr, r, B.N);
-    MPSG_CUDA(cudaGetLastError());
-    ctx->kernel_launches += 2;
+    ob.push_back(OutBlock{B.U, B.S, B.V, R.u.data() + mu.off[iu], R.s.data() + ms.off[is],
+                          R.v.data() + mv.off[iv], B.M, B.N, r});
   }
+  TableImage img;
+  img.add(ob);
+  unsigned char* d = img.upload(ctx->stream);
+  int64_t most = 1;
+  for (const OutBlock& o : ob) most = std::max(most, (o.M + o.N) * o.r);
+  const unsigned gx = (unsigned)std::min<int64_t>((most + 1023) / 1024, 64);
+  svd_outputs_kernel<<<dim3(gx, (unsigned)ob.size()), 256, 0, ctx->stream>>>((OutBlock*)d);
+  MPSG_CUDA(cudaGetLastError());
+  ctx->kernel_launches++;
+  MPSG_CUDA(cudaFreeAsync(d, ctx->stream));
   return R;
 }
 
