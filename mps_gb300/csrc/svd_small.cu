@@ -117,11 +117,12 @@ __device__ __forceinline__ double tangent(double df, double g, int eg, float fg)
 }
 
 // The left singular vectors of columns `order[first], order[first + step], ..`: the reflectors on
-// (V[:, c]; 0), eight lanes a column, NR elements of it in each. z: the cluster's rotated columns.
+// unit[c] (V[:, c]; 0), eight lanes a column, NR elements of it in each. z: the cluster's rotated columns.
 template <int NR>
 __device__ __forceinline__ void left_vectors(double* left, int m, int n, int rank, int first, int step,
                                              double* const* z, const Layout& y, const double* H,
-                                             const double* fac, const int* col, const int* order) {
+                                             const double* fac, const double* unit, const int* col,
+                                             const int* order) {
   const int t = threadIdx.x, l8 = t & 7, C = step;
   for (int j0 = 0; first + step * j0 < n; j0 += kThreads / 8) {
     const int jw = first + step * (j0 + (t >> 5) * 4), j = first + step * (j0 + (t >> 3));
@@ -131,7 +132,7 @@ __device__ __forceinline__ void left_vectors(double* left, int m, int n, int ran
 #pragma unroll
     for (int i = 0; i < NR; ++i) {
       const int r = l8 + 8 * i;
-      x[i] = r < n ? z[r % C][c * y.ld + y.nl + r / C] : 0.0;
+      x[i] = r < n ? z[r % C][c * y.ld + y.nl + r / C] * unit[c] : 0.0;
     }
     for (int k = rank - 1; k >= 0; --k) {
       const double* v = H + col[k] * y.lh;
@@ -416,14 +417,31 @@ __global__ void __launch_bounds__(kThreads) jacobi_svd_kernel(
     if (t == 0) *B.info = 1;
     return;
   }
-  // descending order (d holds the squared norms of the last, rotation-free sweep)
+  // The rotations' rounding has moved the norms of V's columns by some eps: squared norms again, and the
+  // factors (ta) that bring them, and with them the singular values, back.
+  {
+    const int c = t >> 3, end = c < n ? nl : 0;
+    const double* v = Z + c * ld + nl;
+    double s = 0.0;
+    for (int r = l8; r < end; r += 8) s = fma(v[r], v[r], s);
+    for (int o = 4; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (c < ne && l8 < C) z[l8][norms - sm + me * ne + c] = s;
+  }
+  sync();
+  // singular values (d holds the squared norms of the last, rotation-free sweep), descending order
+  if (t < n) {
+    double v = norms[t];
+    for (int q = 1; q < C; ++q) v += norms[q * ne + t];
+    ta[t] = fma(-0.5, v, 1.5);
+    const double s = sqrt(d[t]);
+    isc[t] = 1.0 / s;
+    sc[t] = s * ta[t] * (zero ? 0.0 : __hiloint2double((1023 + ex) << 20, 0));
+  }
+  __syncthreads();
   if (t < n) {
     int at = 0;
-    for (int i = 0; i < n; ++i) at += d[i] > d[t] || (d[i] == d[t] && i < t);
+    for (int i = 0; i < n; ++i) at += sc[i] > sc[t] || (sc[i] == sc[t] && i < t);
     order[at] = t;
-    const double s = sqrt(d[t]);
-    sc[t] = s * (zero ? 0.0 : __hiloint2double((1023 + ex) << 20, 0));
-    isc[t] = 1.0 / s;
   }
   __syncthreads();
   double* left = wide ? B.V : B.U;
@@ -433,9 +451,9 @@ __global__ void __launch_bounds__(kThreads) jacobi_svd_kernel(
     const int j = e / nl, i = e - j * nl, c = order[j];
     if (i * C + me < n) right[col[i * C + me] + (int64_t)j * n] = Z[c * ld + i] * isc[c];
   }
-  if (m <= 64) left_vectors<8>(left, m, n, rank, me, C, z, y, H, fac, col, order);
-  else if (m <= 128) left_vectors<16>(left, m, n, rank, me, C, z, y, H, fac, col, order);
-  else left_vectors<32>(left, m, n, rank, me, C, z, y, H, fac, col, order);
+  if (m <= 64) left_vectors<8>(left, m, n, rank, me, C, z, y, H, fac, ta, col, order);
+  else if (m <= 128) left_vectors<16>(left, m, n, rank, me, C, z, y, H, fac, ta, col, order);
+  else left_vectors<32>(left, m, n, rank, me, C, z, y, H, fac, ta, col, order);
   if (C > 1) cluster.sync();  // its columns may still be read
 }
 
