@@ -282,8 +282,7 @@ __global__ void __launch_bounds__(256) pack_f64_kernel(
   __shared__ uint32_t red[8][33], rlow[8][33];  // largest high words, all low words or-ed
   __shared__ uint2 rmax[kRowBlock];
   __shared__ int rexp[kRowBlock];
-  if (blockIdx.x == 0)  // the GEMM's arrival counters
-    for (int i = threadIdx.x; i < nslots; i += blockDim.x) arrivals[i] = 0;
+  cudaTriggerProgrammaticLaunchCompletion();
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
   const int rank = blockIdx.x % ncta;
   const int2 item = items[blockIdx.x / ncta];
@@ -302,6 +301,9 @@ __global__ void __launch_bounds__(256) pack_f64_kernel(
   const int s0 = min(rank * per, P.nk), s1 = min(s0 + per, P.nk);
   const int64_t kb = (int64_t)s0 * BK, ke = min((int64_t)s1 * BK, K);
   const bool keep = per <= cache_steps;
+  cudaGridDependencySynchronize();
+  if (blockIdx.x == 0)  // the GEMM's arrival counters
+    for (int i = t; i < nslots; i += blockDim.x) arrivals[i] = 0;
   // largest |x| of each row's part: lanes along whichever axis is contiguous
   if (side ? P.fastB : P.fastA) {
     uint32_t m = 0, lo = 0;
@@ -503,6 +505,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f64tc_kernel(
     fence_barrier_init();
   }
   if (warp == 1) tmem_alloc(tmem_slot, kTmemCols);
+  cudaTriggerProgrammaticLaunchCompletion();
+  cudaGridDependencySynchronize();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -969,30 +973,16 @@ static void launch_group(Context* ctx, Group& G, unsigned char* mem, const doubl
     const int smem = steps * BK * kPadRows * (int)sizeof(double);
     set_smem_limit_once(ctx, pack_set, pack_f64_kernel<MAP>,
                         kCacheSteps * BK * kPadRows * (int)sizeof(double));
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)G.nitems * (unsigned)ncta);
-    cfg.blockDim = dim3(256);
-    cfg.dynamicSmemBytes = (size_t)smem;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)ncta;
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = ncta > 1 ? 1 : 0;
-    MPSG_CUDA(cudaLaunchKernelEx(&cfg, pack_f64_kernel<MAP>, (const Problem*)G.d_probs,
-                                 (const int2*)G.d_items, ncta, steps,
-                                 (const AxisEntry*)G.d_axes, (const MapBlock*)G.d_blocks, A, B, RA,
-                                 RB, packA, packB, G.rowsA, G.rowsB, arrivals,
-                                 (int)G.nslots));
+    launch_chained(pack_f64_kernel<MAP>, dim3((unsigned)G.nitems * (unsigned)ncta), dim3(256),
+                   (size_t)smem, st, ncta, G.d_probs, G.d_items, ncta, steps, G.d_axes, G.d_blocks,
+                   A, B, RA, RB, packA, packB, G.rowsA, G.rowsB, arrivals, (int)G.nslots);
     ctx->kernel_launches++;
   }
   KernelTimer timer(ctx, kKindGemmF64, G.flops);
   const int grid = (int)std::min<int64_t>(G.ntiles, ctx->num_sms);
-  gemm_f64tc_kernel<MAP><<<grid, kThreads, kSmemBytes, st>>>(
-      tmA, tmB, G.d_probs, G.d_tiles, G.ntiles, RA, RB, G.d_axes, G.d_blocks, A, B, C, slots,
-      arrivals, ctx->d_tc_err);
-  MPSG_CUDA(cudaGetLastError());
+  launch_chained(gemm_f64tc_kernel<MAP>, dim3((unsigned)grid), dim3(kThreads), (size_t)kSmemBytes, st,
+                 1, tmA, tmB, G.d_probs, G.d_tiles, G.ntiles, RA, RB, G.d_axes, G.d_blocks, A, B, C,
+                 slots, arrivals, ctx->d_tc_err);
   ctx->kernel_launches++;
 }
 

@@ -42,6 +42,8 @@ __global__ void __launch_bounds__(128) contract_small_kernel(
     const MapBlock* __restrict__ blocks, const double* __restrict__ A,
     const double* __restrict__ B, double* __restrict__ C) {
   const int4* ax = reinterpret_cast<const int4*>(axes);
+  cudaTriggerProgrammaticLaunchCompletion();
+  bool waited = false;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total;
        e += (int64_t)gridDim.x * blockDim.x) {
     int lo = 0, hi = nprob - 1;
@@ -58,6 +60,8 @@ __global__ void __launch_bounds__(128) contract_small_kernel(
     const MapBlock* ta = blocks + P.blkA + (me.x & kComboMask) * nkc;
     const MapBlock* tb = blocks + P.blkB + (ne.x & kComboMask) * nkc;
     const int4* ke = ax + P.axK;
+    if (!waited) cudaGridDependencySynchronize();
+    waited = true;
     double acc = 0.0;
     for (int c = 0; c < nkc; ++c) {
       const int2 kc = __ldg(kcombos + P.kc0 + c);
@@ -189,12 +193,14 @@ __global__ void __launch_bounds__(256) contract_thin_kernel(
     double* __restrict__ C) {
   __shared__ ThinShared s;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  cudaTriggerProgrammaticLaunchCompletion();
   for (int it = blockIdx.x; it < nunits; it += gridDim.x) {
     const ThinUnit u = units[it];
     const double* L = u.longB ? B : A;
     const double* S = u.longB ? A : B;
     __syncthreads();  // the previous unit has been read
     if (threadIdx.x < u.K + u.T) s.o[threadIdx.x] = offs[u.offs + threadIdx.x];
+    if (it == blockIdx.x) cudaGridDependencySynchronize();
     for (int x = threadIdx.x; x < u.T * u.K; x += blockDim.x)
       s.b[x] = __ldg(S + __ldg(vals + u.vals + x));
     __syncthreads();
@@ -377,10 +383,8 @@ bool launch_direct(Context* ctx, DirectPlan& p, const double* A, const double* B
     KernelTimer timer(ctx, kKindGemmF64, p.flops - p.tc_flops);
     if (p.elements) {
       const int64_t grid = std::min<int64_t>((p.elements + 127) / 128, (int64_t)ctx->num_sms * 16);
-      contract_small_kernel<<<(unsigned)grid, 128, 0, st>>>(p.d_small, p.nsmall, p.elements,
-                                                           p.d_kcombos, p.d_axes, p.d_blocks, A,
-                                                           B, C);
-      MPSG_CUDA(cudaGetLastError());
+      launch_chained(contract_small_kernel, dim3((unsigned)grid), dim3(128), 0, st, 1, p.d_small,
+                     p.nsmall, p.elements, p.d_kcombos, p.d_axes, p.d_blocks, A, B, C);
       ctx->kernel_launches++;
     }
     if (p.nunits) {
@@ -390,8 +394,8 @@ bool launch_direct(Context* ctx, DirectPlan& p, const double* A, const double* B
                   : p.thin_k <= 16 ? contract_thin_kernel<16, 1>
                                    : contract_thin_kernel<32, 1>;
       const int grid = std::min(p.nunits, ctx->num_sms * 8);
-      kern<<<grid, 256, 0, st>>>(p.d_units, p.nunits, p.d_offs, p.d_vals, A, B, C);
-      MPSG_CUDA(cudaGetLastError());
+      launch_chained(kern, dim3((unsigned)grid), dim3(256), 0, st, 1, p.d_units, p.nunits, p.d_offs,
+                     p.d_vals, A, B, C);
       ctx->kernel_launches++;
     }
   }

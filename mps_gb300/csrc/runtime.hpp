@@ -26,6 +26,31 @@ namespace mpsg {
       throw ::mpsg::Error(::mpsg::kErrCuda, std::string(#call) + ": " + cudaGetErrorString(e_)); \
   } while (0)
 
+// Launches a kernel that may start while the previous kernel of the stream ends: its blocks set up, read
+// tables uploaded before that kernel and call cudaGridDependencySynchronize() before they touch anything
+// else, every block of them (so that one kernel's end implies the end of all before it). Kernels
+// launched so also let their successor start (cudaTriggerProgrammaticLaunchCompletion).
+// Measured with the launches of a contraction chained so, two-site H_eff: chi = 48 42 -> 30 us (4 launches),
+// chi = 517 122 -> 114 us (6), a chi = 64 DMRG sweep of 32 sites 112 -> 99 ms.
+template <class... P, class... A>
+void launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                    int cluster, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = (unsigned)cluster;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  MPSG_CUDA(cudaLaunchKernelEx(&cfg, kernel, P(args)...));
+}
+
 struct Context;
 struct HeffPlans;
 namespace split {
