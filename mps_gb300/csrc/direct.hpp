@@ -9,10 +9,10 @@ namespace mpsg {
 
 // One sector GEMM of the element-per-thread kernel (block tables as in MapProblem).
 struct SmallProblem {
-  int64_t first;             // first element (row fastest) of the launch
-  int32_t M, N;
+  int32_t first, mt;         // first tile (rows fastest) of the launch, tiles along the rows
+  int32_t M, N, K;
   int32_t axM, axN, axK;     // first axis entries
-  int32_t kc0, nkc, nnc;     // k combos, their count, column combos
+  int32_t nkc, nnc;          // k combos, column combos
   int32_t blkA, blkB, blkC;  // first blocks
 };
 
@@ -37,13 +37,12 @@ constexpr int kThinMax = 32;
 
 struct DirectTables {
   std::vector<SmallProblem> small;
-  std::vector<int2> kcombos;  // (first k, count)
   std::vector<ThinUnit> units;
   std::vector<ThinOffset> offs;
   std::vector<int64_t> vals;
   std::vector<AxisEntry> axes;
   std::vector<MapBlock> blocks;
-  int64_t elements = 0;           // of the small problems
+  int64_t small_tiles = 0;        // of the small problems
   std::vector<f64tc::Task> tiled; // points into the map it was planned from
 };
 
@@ -51,14 +50,12 @@ struct DirectPlan {
   unsigned char* d_tables = nullptr;
   cudaStream_t stream = nullptr;
   SmallProblem* d_small = nullptr;
-  int2* d_kcombos = nullptr;
   ThinUnit* d_units = nullptr;
   ThinOffset* d_offs = nullptr;
   int64_t* d_vals = nullptr;
   AxisEntry* d_axes = nullptr;
   MapBlock* d_blocks = nullptr;
-  int nsmall = 0, nunits = 0, thin_k = 0;
-  int64_t elements = 0;
+  int nsmall = 0, small_tiles = 0, nunits = 0, thin_k = 0;
   double flops = 0, tc_flops = 0;
   std::unique_ptr<f64tc::Plan> tc;
   // false: the contraction cannot be mapped, or the fused path is the better one for it

@@ -31,51 +31,98 @@ __device__ __forceinline__ int col_part(const BlockRegs& b, const int4& e) {
   return e.y * b.cs0 + e.z * b.cs1 + e.w * b.cs2;
 }
 
-// One thread per result element, every sector GEMM of a small contraction in one launch. Bound by
-// latency: the chain of a thread is K dependent FMAs behind prefetched loads, so what counts is
-// that the elements spread over the whole chip (a 64 x 64 tile kernel keeps them on a few SMs, each
-// at 2 FMAs per cycle) and that nothing runs before or after it. Measured, the four contractions of
-// a chi = 48 two-site H_eff: 4 launches of 7.3 us against 19 of 205 us in all.
-__global__ void __launch_bounds__(128) contract_small_kernel(
-    const SmallProblem* __restrict__ probs, int nprob, int64_t total,
-    const int2* __restrict__ kcombos, const AxisEntry* __restrict__ axes,
-    const MapBlock* __restrict__ blocks, const double* __restrict__ A,
-    const double* __restrict__ B, double* __restrict__ C) {
+// Every sector GEMM of a small contraction in one launch: a CTA takes 32 rows and 4 columns of a result,
+// one element per thread, its operands staged in shared memory kChunk contracted indices at a
+// time. Bound by latency: what counts is that the elements spread over the whole chip (a 64 x 64 tile
+// kernel keeps them on a few SMs, each at 2 FMAs per cycle), that the loads of an element's sum do
+// not wait for one another (all of a CTA's are issued at once, index tables first; as a loop of
+// each thread they took 15 of the last contraction's 17 us) and that nothing runs before or after it.
+// Measured, the four contractions of a chi = 48 two-site H_eff: 26.6 us with the gaps between them (29.7 us as thread loops) against
+// 19 launches of 205 us in all.
+constexpr int kChunk = 128, kSmallRows = 32, kSmallCols = 4;
+
+// Offset of a row's (or column's) element at contracted index x, through its block table.
+__device__ __forceinline__ int64_t mapped_at(const MapBlock* __restrict__ tab, const int4& row,
+                                             const int4& x) {
+  const BlockRegs b = load_block(tab + (x.x & kComboMask));
+  return row_part(b, row) + col_part(b, x);
+}
+
+__global__ void __launch_bounds__(kSmallRows * kSmallCols) contract_small_kernel(
+    const SmallProblem* __restrict__ probs, int nprob, int ntiles,
+    const AxisEntry* __restrict__ axes, const MapBlock* __restrict__ blocks,
+    const double* __restrict__ A, const double* __restrict__ B, double* __restrict__ C) {
+  __shared__ double as[kChunk * kSmallRows], bs[kChunk * kSmallCols];
   const int4* ax = reinterpret_cast<const int4*>(axes);
+  const int t = threadIdx.x, lane = t & 31, w = t >> 5;
   cudaTriggerProgrammaticLaunchCompletion();
-  bool waited = false;
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total;
-       e += (int64_t)gridDim.x * blockDim.x) {
+  for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
     int lo = 0, hi = nprob - 1;
     while (lo < hi) {
       const int mid = (lo + hi + 1) >> 1;
-      if (__ldg(&probs[mid].first) <= e) lo = mid;
+      if (__ldg(&probs[mid].first) <= tile) lo = mid;
       else hi = mid - 1;
     }
-    const SmallProblem& P = probs[lo];
-    const uint32_t lt = (uint32_t)(e - P.first);
-    const uint32_t j = lt / (uint32_t)P.M, i = lt - j * (uint32_t)P.M;
-    const int4 me = __ldg(ax + P.axM + i), ne = __ldg(ax + P.axN + j);
-    const int nkc = P.nkc;
-    const MapBlock* ta = blocks + P.blkA + (me.x & kComboMask) * nkc;
-    const MapBlock* tb = blocks + P.blkB + (ne.x & kComboMask) * nkc;
-    const int4* ke = ax + P.axK;
-    if (!waited) cudaGridDependencySynchronize();
-    waited = true;
+    const SmallProblem P = probs[lo];
+    const int ni = (tile - P.first) / P.mt, mi = tile - P.first - ni * P.mt;
+    const int i = mi * kSmallRows + lane, j = ni * kSmallCols + w;
+    const int4 me = __ldg(ax + P.axM + min(i, P.M - 1)), ne = __ldg(ax + P.axN + min(j, P.N - 1));
+    const int4 nl = __ldg(ax + P.axN + min(ni * kSmallCols + (t & 3), P.N - 1));  // column it stages
+    const MapBlock* ta = blocks + P.blkA + (me.x & kComboMask) * P.nkc;
+    const MapBlock* tb = blocks + P.blkB + (nl.x & kComboMask) * P.nkc;
+    const BlockRegs bc =
+        load_block(blocks + P.blkC + (me.x & kComboMask) * P.nnc + (ne.x & kComboMask));
     double acc = 0.0;
-    for (int c = 0; c < nkc; ++c) {
-      const int2 kc = __ldg(kcombos + P.kc0 + c);
-      const BlockRegs ba = load_block(ta + c), bb = load_block(tb + c);
-      const double* pa = A + row_part(ba, me);
-      const double* pb = B + row_part(bb, ne);
-#pragma unroll 8
-      for (int k = 0; k < kc.y; ++k) {
-        const int4 x = __ldg(ke + kc.x + k);
-        acc = fma(__ldg(pa + col_part(ba, x)), __ldg(pb + col_part(bb, x)), acc);
+    for (int c0 = 0; c0 == 0 || c0 < P.K; c0 += kChunk) {
+      const int4* ke = ax + P.axK + c0;
+      const int kn = min(kChunk, P.K - c0);
+      constexpr int kPart = kChunk / 2, kA = kPart / kSmallCols, kB = kChunk / kSmallRows;
+      int64_t oa[kA], ob[kB];  // all addresses, then all loads
+#pragma unroll
+      for (int u = 0; u < kB; ++u) {
+        const int k = (t >> 2) + kSmallRows * u;
+        if (k < kn) ob[u] = mapped_at(tb, nl, __ldg(ke + k));
       }
+#pragma unroll
+      for (int u = 0; u < kA; ++u) {
+        const int k = w + kSmallCols * u;
+        if (k < kn) oa[u] = mapped_at(ta, me, __ldg(ke + k));
+      }
+      if (tile == blockIdx.x && c0 == 0) cudaGridDependencySynchronize();
+      double va[kA], vb[kB];
+#pragma unroll
+      for (int u = 0; u < kB; ++u)
+        if ((t >> 2) + kSmallRows * u < kn) vb[u] = __ldg(B + ob[u]);
+#pragma unroll
+      for (int u = 0; u < kA; ++u)
+        if (w + kSmallCols * u < kn) va[u] = __ldg(A + oa[u]);
+      if (c0 > 0 || tile != blockIdx.x) __syncthreads();  // the last chunk has been read
+#pragma unroll
+      for (int u = 0; u < kA; ++u)
+        if (w + kSmallCols * u < kn) as[(w + kSmallCols * u) * kSmallRows + lane] = va[u];
+      if (kn > kPart) {
+#pragma unroll
+        for (int u = 0; u < kA; ++u) {
+          const int k = kPart + w + kSmallCols * u;
+          if (k < kn) va[u] = __ldg(A + mapped_at(ta, me, __ldg(ke + k)));
+        }
+#pragma unroll
+        for (int u = 0; u < kA; ++u) {
+          const int k = kPart + w + kSmallCols * u;
+          if (k < kn) as[k * kSmallRows + lane] = va[u];
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < kB; ++u) {
+        const int k = (t >> 2) + kSmallRows * u;
+        if (k < kn) bs[k * kSmallCols + (t & 3)] = vb[u];
+      }
+      __syncthreads();
+#pragma unroll 8
+      for (int k = 0; k < kn; ++k)
+        acc = fma(as[k * kSmallRows + lane], bs[k * kSmallCols + w], acc);
     }
-    const BlockRegs bc = load_block(blocks + P.blkC + (me.x & kComboMask) * P.nnc + (ne.x & kComboMask));
-    C[row_part(bc, me) + col_part(bc, ne)] = acc;
+    if (i < P.M && j < P.N) C[row_part(bc, me) + col_part(bc, ne)] = acc;
   }
 }
 
@@ -265,21 +312,21 @@ void plan_direct(const std::vector<MapProblem>& map, const std::vector<GemmTask>
       return at;
     };
     if (small) {
-      SmallProblem s;
-      s.first = t.elements;
+      SmallProblem s{};
+      s.first = (int32_t)t.small_tiles;
       s.M = (int32_t)q.M;
       s.N = (int32_t)q.N;
+      s.K = (int32_t)q.K;
+      s.mt = (int32_t)((q.M + kSmallRows - 1) / kSmallRows);
       s.axM = axis(q.m);
       s.axN = axis(q.n);
       s.axK = axis(q.k);
-      s.kc0 = (int32_t)t.kcombos.size();
       s.nkc = (int32_t)q.k.size();
       s.nnc = (int32_t)q.n.size();
-      for (const AxisCombo& c : q.k) t.kcombos.push_back(make_int2(c.start, c.count));
       s.blkA = table(q.A);
       s.blkB = table(q.B);
       s.blkC = table(q.C);
-      t.elements += q.M * q.N;
+      t.small_tiles += s.mt * ((q.N + kSmallCols - 1) / kSmallCols);
       t.small.push_back(s);
     } else if (q.K <= kThinMax && std::min(q.M, q.N) <= kThinMax &&
                !(tiled && std::max(q.M, q.N) <= kTiledThin)) {
@@ -351,11 +398,9 @@ bool DirectPlan::build(const ContractPlan& p, const TensorMeta& A, const TensorM
   flops = p.flops;
   for (const auto& x : t.tiled) tc_flops += 2.0 * x.g.M * x.g.N * x.g.K;
   TableImage img;
-  const size_t os = img.add(t.small), ok = img.add(t.kcombos),
-               ou = img.add(t.units), of = img.add(t.offs), ov = img.add(t.vals), oa = img.add(t.axes), ob = img.add(t.blocks);
+  const size_t os = img.add(t.small), ou = img.add(t.units), of = img.add(t.offs), ov = img.add(t.vals), oa = img.add(t.axes), ob = img.add(t.blocks);
   d_tables = img.upload(st);
   d_small = (SmallProblem*)(d_tables + os);
-  d_kcombos = (int2*)(d_tables + ok);
   d_units = (ThinUnit*)(d_tables + ou);
   d_offs = (ThinOffset*)(d_tables + of);
   d_vals = (int64_t*)(d_tables + ov);
@@ -363,7 +408,7 @@ bool DirectPlan::build(const ContractPlan& p, const TensorMeta& A, const TensorM
   d_blocks = (MapBlock*)(d_tables + ob);
   nsmall = (int)t.small.size();
   nunits = (int)t.units.size();
-  elements = t.elements;
+  small_tiles = (int)t.small_tiles;
   for (const ThinUnit& x : t.units) thin_k = std::max(thin_k, x.K);
   if (!t.tiled.empty()) {
     tc = std::make_unique<f64tc::Plan>();
@@ -379,12 +424,12 @@ DirectPlan::~DirectPlan() {
 bool launch_direct(Context* ctx, DirectPlan& p, const double* A, const double* B, double* C) {
   cudaStream_t st = ctx->stream;
   if (p.tc && !f64tc::launch(ctx, *p.tc, A, B, C)) return false;
-  if (p.elements || p.nunits) {
+  if (p.small_tiles || p.nunits) {
     KernelTimer timer(ctx, kKindGemmF64, p.flops - p.tc_flops);
-    if (p.elements) {
-      const int64_t grid = std::min<int64_t>((p.elements + 127) / 128, (int64_t)ctx->num_sms * 16);
-      launch_chained(contract_small_kernel, dim3((unsigned)grid), dim3(128), 0, st, 1, p.d_small,
-                     p.nsmall, p.elements, p.d_kcombos, p.d_axes, p.d_blocks, A, B, C);
+    if (p.small_tiles) {
+      const int grid = std::min(p.small_tiles, ctx->num_sms * 16);
+      launch_chained(contract_small_kernel, dim3((unsigned)grid), dim3(kSmallRows * kSmallCols), 0, st,
+                     1, p.d_small, p.nsmall, p.small_tiles, p.d_axes, p.d_blocks, A, B, C);
       ctx->kernel_launches++;
     }
     if (p.nunits) {
