@@ -442,6 +442,15 @@ int mpsg_contract_complex(mpsg_ctx* ctx, const mpsg_tensor* ar, const mpsg_tenso
     mpsg::Context* c = &ctx->c;
     const auto ia = ivec(idxa, ar->t.meta.N());
     const auto ib = ivec(idxb, br->t.meta.N());
+    {
+      mpsg::DeviceTensor re, im;
+      if (mpsg::contract_complex(c, ar->t, ai ? &ai->t : nullptr, sa, ia, br->t,
+                                 bi ? &bi->t : nullptr, sb, ib, precision, re, im)) {
+        *cr = wrap(std::move(re));
+        *ci = wrap(std::move(im));
+        return;
+      }
+    }
     double srr = 0, sri = 0, sir = 0, sii = 0;
     mpsg::DeviceTensor rr = mpsg::contract(c, ar->t, ia, br->t, ib, precision, &srr);
     mpsg::DeviceTensor ri, ir, ii;

@@ -141,6 +141,52 @@ void append_axis(const std::vector<AxisCombo>& combos, std::vector<AxisEntry>& o
   }
 }
 
+std::vector<MapProblem> complex_map(const std::vector<MapProblem>& map, bool ca, bool cb) {
+  std::vector<MapProblem> out;
+  auto twice = [](std::vector<AxisCombo>& axis, int64_t n) {
+    const size_t k = axis.size();
+    for (size_t i = 0; i < k; ++i) {
+      axis.push_back(axis[i]);
+      axis.back().start += (int32_t)n;
+    }
+  };
+  auto with_part = [](std::vector<MapBlock>& t) {
+    const size_t k = t.size();
+    for (size_t i = 0; i < k; ++i) {
+      t.push_back(t[i]);
+      t.back().base |= (int64_t)1 << kPartShift;
+    }
+  };
+  for (MapProblem q : map) {
+    const size_t nm = q.m.size(), nn = q.n.size();
+    const std::vector<MapBlock> c = q.C;
+    const int pa = ca ? 2 : 1, pb = cb ? 2 : 1;
+    if (q.M * pa > INT32_MAX || q.N * pb > INT32_MAX ||
+        std::max(nm * pa, nn * pb) > (size_t)kComboMask)
+      return {};
+    q.C.clear();
+    for (int x = 0; x < pa; ++x)
+      for (size_t i = 0; i < nm; ++i)
+        for (int y = 0; y < pb; ++y)
+          for (size_t j = 0; j < nn; ++j) {
+            q.C.push_back(c[i * nn + j]);
+            q.C.back().base |= (int64_t)(x * pb + y) << kPartShift;
+          }
+    if (ca) {
+      twice(q.m, q.M);
+      with_part(q.A);
+      q.M *= 2;
+    }
+    if (cb) {
+      twice(q.n, q.N);
+      with_part(q.B);
+      q.N *= 2;
+    }
+    out.push_back(std::move(q));
+  }
+  return out;
+}
+
 std::vector<MapProblem> build_contract_map(const ContractPlan& p, const TensorMeta& A,
                                            const TensorMeta& B) {
   std::vector<MapProblem> none;

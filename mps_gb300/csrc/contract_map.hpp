@@ -52,6 +52,29 @@ struct MapProblem {
 std::vector<MapProblem> build_contract_map(const ContractPlan& p, const TensorMeta& A,
                                            const TensorMeta& B);
 
+// Bits of a block's base that name the tensor it is in, where an operand or the result is several
+// tensors of one structure (real and imaginary parts): part 0 has the pointer of a launch, the
+// others are at distances (in elements) given with it.
+constexpr int kPartShift = 61;
+struct PartOffsets {
+  int64_t a = 0, b = 0;          // from the real to the imaginary part of A, of B
+  int64_t c1 = 0, c2 = 0, c3 = 0;  // from part 0 of the result to the others
+};
+
+// The map of the products of all parts of A and B, in the parts of A that have an imaginary one (ca)
+// stacked along the rows and those of B (cb) along the columns. Part of the result: 2 [imaginary part of
+// A] + [imaginary part of B] for two complex operands, else the part of the complex one.
+// Empty when an axis gets too long.
+std::vector<MapProblem> complex_map(const std::vector<MapProblem>& map, bool ca, bool cb);
+
+#ifdef __CUDACC__
+__device__ __forceinline__ int64_t part_base(int64_t base, int64_t d1, int64_t d2, int64_t d3) {
+  const int part = (int)(base >> kPartShift);
+  if (part) base = (base & (((int64_t)1 << kPartShift) - 1)) + (part == 1 ? d1 : part == 2 ? d2 : d3);
+  return base;
+}
+#endif
+
 // Appends the entries of an axis.
 void append_axis(const std::vector<AxisCombo>& combos, std::vector<AxisEntry>& out);
 

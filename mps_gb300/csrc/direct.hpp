@@ -59,8 +59,9 @@ struct DirectPlan {
   double flops = 0, tc_flops = 0;
   std::unique_ptr<f64tc::Plan> tc;
   // false: the contraction cannot be mapped, or the fused path is the better one for it
+  // ca, cb: A, B have imaginary parts (the products of all parts in one set of launches)
   bool build(const ContractPlan& p, const TensorMeta& A, const TensorMeta& B, int num_sms,
-             cudaStream_t st);
+             cudaStream_t st, bool ca, bool cb);
   ~DirectPlan();
 };
 
@@ -70,6 +71,11 @@ void plan_direct(const std::vector<MapProblem>& map, const std::vector<GemmTask>
 
 // C = contract(A, B); false (nothing useful written) when scratch for the tensor cores could not be
 // had.
-bool launch_direct(Context* ctx, DirectPlan& p, const double* A, const double* B, double* C);
+bool launch_direct(Context* ctx, DirectPlan& p, const double* A, const double* B, double* C,
+                   const PartOffsets& parts = PartOffsets());
+
+// re = rr + c_ii ii in place of rr, im = c_ri ri + c_ir ir in place of ri
+void launch_complex_parts(Context* ctx, int64_t n, double* rr, double* ri, const double* ir,
+                          const double* ii, double c_ri, double c_ir, double c_ii);
 
 }  // namespace mpsg

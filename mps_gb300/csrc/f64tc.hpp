@@ -88,7 +88,8 @@ bool eligible(const GemmTask& t);
 // C = A B for every problem of the plan. A plan whose operands are fused matrices falls back on the
 // FP64 pipe where the packed operands find no memory; a mapped one returns false then, with
 // nothing written that a rerun would not write again.
-bool launch(Context* ctx, Plan& p, const double* A, const double* B, double* C);
+bool launch(Context* ctx, Plan& p, const double* A, const double* B, double* C,
+            const PartOffsets& parts = PartOffsets());
 
 }  // namespace f64tc
 }  // namespace mpsg

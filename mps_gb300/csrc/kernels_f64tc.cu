@@ -45,6 +45,7 @@
 #include <cuda_bf16.h>
 
 #include <algorithm>
+#include <type_traits>
 
 #include "f64tc.hpp"
 #include "tc5.cuh"
@@ -200,13 +201,29 @@ __device__ __forceinline__ AxisEntry load_entry(const AxisEntry* e) {
 
 constexpr int kRun = 8;  // elements that run8 fetches
 
+// How a kernel finds elements: by strides (kFused), through block tables (kMapped), or through block
+// tables that name one of several tensors (kParts).
+enum Access { kFused, kMapped, kParts };
+
+// Base of a block, with the distance of the part it is in.
+template <bool PARTS>
+struct PartBase {
+  __device__ __forceinline__ PartBase(int64_t, int64_t, int64_t) {}
+  __device__ __forceinline__ int64_t of(int64_t base) const { return base; }
+};
+template <>
+struct PartBase<true> {
+  int64_t p1, p2, p3;
+  __device__ __forceinline__ PartBase(int64_t a, int64_t b, int64_t c) : p1(a), p2(b), p3(c) {}
+  __device__ __forceinline__ int64_t of(int64_t base) const { return part_base(base, p1, p2, p3); }
+};
+
 // Addresses along one row of an operand or of the output: strided, or through the block table row
 // `tab` of the row's combo (a new block is looked up when the column's combo changes).
-template <bool MAP>
-struct Cursor {
+struct FusedCursor {
   int64_t at0, step;
-  __device__ __forceinline__ Cursor(const MapBlock*, const AxisEntry*, int64_t o, int64_t row,
-                                    int64_t rs, int64_t cs)
+  __device__ __forceinline__ FusedCursor(const MapBlock*, const AxisEntry*, int64_t o, int64_t row,
+                                         int64_t rs, int64_t cs, int64_t, int64_t = 0, int64_t = 0)
       : at0(o + row * rs), step(cs) {}
   __device__ __forceinline__ int64_t at(const AxisEntry*, int64_t col) { return at0 + col * step; }
   // x[j] = X[element col + j], zero from column `end` on
@@ -218,15 +235,19 @@ struct Cursor {
   }
 };
 
-template <>
-struct Cursor<true> {
+template <bool PARTS>
+struct MapCursor {
   const MapBlock* tab;
   AxisEntry r;
   int combo = -1, row = 0, c0 = 0, c1 = 0, c2 = 0;
   int64_t base = 0;
-  // tab: the table's first block, ncol blocks per row combo; entry: the row's axis entry
-  __device__ __forceinline__ Cursor(const MapBlock* t, const AxisEntry* entry, int64_t, int64_t,
-                                    int64_t, int64_t ncol) {
+  PartBase<PARTS> parts;
+  // tab: the table's first block, ncol blocks per row combo; entry: the row's axis entry; p1..p3:
+  // distances of the parts
+  __device__ __forceinline__ MapCursor(const MapBlock* t, const AxisEntry* entry, int64_t, int64_t,
+                                       int64_t, int64_t ncol, int64_t p1, int64_t p2 = 0,
+                                       int64_t p3 = 0)
+      : parts(p1, p2, p3) {
     r = load_entry(entry);
     tab = t + (int64_t)(r.combo_run & kComboMask) * ncol;
   }
@@ -238,7 +259,7 @@ struct Cursor<true> {
       combo = e.combo_run & kComboMask;
       const int4* b = reinterpret_cast<const int4*>(tab + combo);
       const int4 x = __ldg(b), y = __ldg(b + 1);
-      base = (int64_t)(((unsigned long long)(unsigned)x.y << 32) | (unsigned)x.x);
+      base = parts.of((int64_t)(((unsigned long long)(unsigned)x.y << 32) | (unsigned)x.x));
       row = r.i[0] * x.z + r.i[1] * x.w + r.i[2] * y.x;
       c0 = y.y;
       c1 = y.z;
@@ -258,11 +279,14 @@ struct Cursor<true> {
     }
     int64_t a[kRun];
 #pragma unroll
-    for (int j = 0; j < kRun; ++j) a[j] = col + j < end ? at(cols, col + j) : -1;
+    for (int j = 0; j < kRun; ++j) a[j] = col + j < end ? at(cols, col + j) : 0;
 #pragma unroll
-    for (int j = 0; j < kRun; ++j) x[j] = a[j] >= 0 ? __ldg(X + a[j]) : 0.0;
+    for (int j = 0; j < kRun; ++j) x[j] = col + j < end ? __ldg(X + a[j]) : 0.0;
   }
 };
+
+template <Access MAP>
+using Cursor = std::conditional_t<MAP == kFused, FusedCursor, MapCursor<MAP == kParts>>;
 
 // One cluster per item (32 rows of one operand, whole K), its K steps shared out over the CTAs: each
 // CTA keeps its part in shared memory while it finds the rows' largest elements, the CTAs exchange
@@ -271,13 +295,14 @@ struct Cursor<true> {
 // 8 x 256) is read again instead of kept.
 constexpr int kCacheSteps = 8, kPadRows = kRowBlock + 1, kMaxCluster = 8;
 
-template <bool MAP>
+template <Access MAP>
 __global__ void __launch_bounds__(256) pack_f64_kernel(
     const Problem* __restrict__ probs, const int2* __restrict__ items, int ncta, int cache_steps,
     const AxisEntry* __restrict__ axes, const MapBlock* __restrict__ blocks,
     const double* __restrict__ A, const double* __restrict__ B, int32_t* __restrict__ RA,
     int32_t* __restrict__ RB, __nv_bfloat16* __restrict__ packA, __nv_bfloat16* __restrict__ packB,
-    int64_t rowsA, int64_t rowsB, int* __restrict__ arrivals, int nslots) {
+    int64_t rowsA, int64_t rowsB, int* __restrict__ arrivals, int nslots, int64_t partA,
+    int64_t partB) {
   extern __shared__ double xs[];  // [k][row], rows padded to kPadRows
   __shared__ uint32_t red[8][33], rlow[8][33];  // largest high words, all low words or-ed
   __shared__ uint2 rmax[kRowBlock];
@@ -292,6 +317,7 @@ __global__ void __launch_bounds__(256) pack_f64_kernel(
   const int64_t rows = side ? P.N : P.M, rs = side ? P.brs : P.ars;
   const int64_t kstep = MAP ? P.nkc : (side ? P.bks : P.aks);
   const double* X = ((P.swap != 0) != (side != 0)) ? B : A;
+  const int64_t part = ((P.swap != 0) != (side != 0)) ? partB : partA;
   const int64_t x0 = side ? P.ob : P.oa;
   const MapBlock* tab = blocks + (side ? P.blkB : P.blkA);
   const AxisEntry* row_ax = axes + (side ? P.axN : P.axM);
@@ -308,7 +334,7 @@ __global__ void __launch_bounds__(256) pack_f64_kernel(
   if (side ? P.fastB : P.fastA) {
     uint32_t m = 0, lo = 0;
     if (lane < nr) {
-      Cursor<MAP> c(tab, row_ax + r0 + lane, x0, r0 + lane, rs, kstep);
+      Cursor<MAP> c(tab, row_ax + r0 + lane, x0, r0 + lane, rs, kstep, part);
       for (int64_t k = kb + w * kRun; k < (int64_t)s1 * BK; k += 8 * kRun) {
         double x[kRun];
         if (k < ke) {
@@ -332,7 +358,7 @@ __global__ void __launch_bounds__(256) pack_f64_kernel(
     for (int rr = w; rr < kRowBlock; rr += 8) {
       uint32_t m = 0, lo = 0;
       if (rr < nr) {
-        Cursor<MAP> c(tab, row_ax + r0 + rr, x0, r0 + rr, rs, kstep);
+        Cursor<MAP> c(tab, row_ax + r0 + rr, x0, r0 + rr, rs, kstep, part);
 #pragma unroll 4
         for (int64_t k = kb + lane; k < ke; k += 32) {
           const double x = __ldg(X + c.at(k_ax, k));
@@ -388,7 +414,7 @@ __global__ void __launch_bounds__(256) pack_f64_kernel(
   const int64_t plane = (side ? rowsB : rowsA) * BK;
   __nv_bfloat16* out = (side ? packB : packA) + (r % rpt) * BK + g8;
   const int e = rexp[rr];
-  Cursor<MAP> c(tab, row_ax + r, x0, r, rs, kstep);
+  Cursor<MAP> c(tab, row_ax + r, x0, r, rs, kstep, part);
   for (int s = s0 + (w >> 2); s < s1; s += 2) {
     const int64_t k0 = (int64_t)s * BK + g8;
     double x[kRun];
@@ -445,17 +471,20 @@ __global__ void __launch_bounds__(256) pack_f64_kernel(
 
 // Output elements n0 .. n0 + nc of one row that are not sliced (the row, or the element's column, is
 // marked): the chain of FP64 FMAs over k.
-template <bool MAP>
+template <Access MAP>
 __device__ __noinline__ void fma_chains(const Problem& P, int64_t row, int64_t n0, int nc,
                                         bool all, const int32_t* RB, const AxisEntry* axes,
                                         const MapBlock* blocks, const double* R, const double* S,
-                                        double* C) {
+                                        double* C, const PartOffsets& parts) {
   const AxisEntry *m_ax = axes + P.axM + row, *n_ax = axes + P.axN, *k_ax = axes + P.axK;
-  Cursor<MAP> out(blocks + P.blkC, m_ax, P.oc, row, P.crs, MAP ? P.nnc : P.ccs);
+  Cursor<MAP> out(blocks + P.blkC, m_ax, P.oc, row, P.crs, MAP ? P.nnc : P.ccs,
+                  parts.c1, parts.c2, parts.c3);
   for (int j = 0; j < nc; ++j) {
     if (!all && RB[j] != kRowBad) continue;
-    Cursor<MAP> a(blocks + P.blkA, m_ax, P.oa, row, P.ars, MAP ? P.nkc : P.aks);
-    Cursor<MAP> b(blocks + P.blkB, n_ax + n0 + j, P.ob, n0 + j, P.brs, MAP ? P.nkc : P.bks);
+    Cursor<MAP> a(blocks + P.blkA, m_ax, P.oa, row, P.ars, MAP ? P.nkc : P.aks,
+                  P.swap ? parts.b : parts.a);
+    Cursor<MAP> b(blocks + P.blkB, n_ax + n0 + j, P.ob, n0 + j, P.brs, MAP ? P.nkc : P.bks,
+                  P.swap ? parts.a : parts.b);
     double y = 0.0;
     for (int64_t k = 0; k < P.K; ++k) y = fma(R[a.at(k_ax, k)], S[b.at(k_ax, k)], y);
     C[out.at(n_ax, n0 + j)] = y;
@@ -468,14 +497,15 @@ constexpr int64_t kSlotLo = (int64_t)BM * BN * 8, kSlotBytes = (int64_t)BM * BN 
 // epilogue warps (five per TMEM lane quarter, 16 columns each). Every mbarrier wait is bounded;
 // on expiry the kernel records an error code, stops issuing, waits for its own MMAs and frees
 // TMEM.
-template <bool MAP>
+template <Access MAP>
 __global__ void __launch_bounds__(kThreads, 1) gemm_f64tc_kernel(
     const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
     const Problem* __restrict__ probs, const Tile* __restrict__ tiles, int64_t ntiles,
     const int32_t* __restrict__ RA, const int32_t* __restrict__ RB,
     const AxisEntry* __restrict__ axes, const MapBlock* __restrict__ blocks,
     const double* __restrict__ A, const double* __restrict__ B, double* __restrict__ C,
-    unsigned char* __restrict__ slots, int* __restrict__ arrivals, int* __restrict__ err) {
+    unsigned char* __restrict__ slots, int* __restrict__ arrivals, int* __restrict__ err,
+    const __grid_constant__ PartOffsets parts) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   uint64_t* bars = (uint64_t*)(smem + kStages * kStageBytes);
@@ -690,7 +720,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f64tc_kernel(
           hi[j] = __double_as_longlong(y);
         }
         Cursor<MAP> out(blocks + P.blkC, axes + P.axM + row, P.oc, row, P.crs,
-                        MAP ? P.nnc : P.ccs);
+                        MAP ? P.nnc : P.ccs, parts.c1, parts.c2, parts.c3);
         const AxisEntry* n_ax = axes + P.axN;
 #pragma unroll
         for (int j = 0; j < kEpiCols; ++j) {
@@ -699,7 +729,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f64tc_kernel(
         }
         if (bad)
           fma_chains<MAP>(P, row, n0, nc, er == kRowBad, RBp, axes, blocks, P.swap ? B : A,
-                          P.swap ? A : B, C);
+                          P.swap ? A : B, C, parts);
       }
     }
   }
@@ -947,9 +977,9 @@ void Plan::release() {
   groups.clear();
 }
 
-template <bool MAP>
+template <Access MAP>
 static void launch_group(Context* ctx, Group& G, unsigned char* mem, const double* A,
-                         const double* B, double* C) {
+                         const double* B, double* C, const PartOffsets& parts) {
   static std::once_flag smem_set[kMaxDevices], pack_set[kMaxDevices];
   cudaStream_t st = ctx->stream;
   const size_t bA = round256((size_t)G.rowsA * BK * 2 * kSlices),
@@ -975,18 +1005,20 @@ static void launch_group(Context* ctx, Group& G, unsigned char* mem, const doubl
                         kCacheSteps * BK * kPadRows * (int)sizeof(double));
     launch_chained(pack_f64_kernel<MAP>, dim3((unsigned)G.nitems * (unsigned)ncta), dim3(256),
                    (size_t)smem, st, ncta, G.d_probs, G.d_items, ncta, steps, G.d_axes, G.d_blocks,
-                   A, B, RA, RB, packA, packB, G.rowsA, G.rowsB, arrivals, (int)G.nslots);
+                   A, B, RA, RB, packA, packB, G.rowsA, G.rowsB, arrivals, (int)G.nslots, parts.a,
+                   parts.b);
     ctx->kernel_launches++;
   }
   KernelTimer timer(ctx, kKindGemmF64, G.flops);
   const int grid = (int)std::min<int64_t>(G.ntiles, ctx->num_sms);
   launch_chained(gemm_f64tc_kernel<MAP>, dim3((unsigned)grid), dim3(kThreads), (size_t)kSmemBytes, st,
                  1, tmA, tmB, G.d_probs, G.d_tiles, G.ntiles, RA, RB, G.d_axes, G.d_blocks, A, B, C,
-                 slots, arrivals, ctx->d_tc_err);
+                 slots, arrivals, ctx->d_tc_err, parts);
   ctx->kernel_launches++;
 }
 
-bool launch(Context* ctx, Plan& p, const double* A, const double* B, double* C) {
+bool launch(Context* ctx, Plan& p, const double* A, const double* B, double* C,
+            const PartOffsets& parts) {
   cudaStream_t st = ctx->stream;
   for (Group& G : p.groups) {
     if (G.ntiles == 0) continue;
@@ -1005,8 +1037,9 @@ bool launch(Context* ctx, Plan& p, const double* A, const double* B, double* C) 
       continue;
     }
     MPSG_CUDA(e);
-    if (p.mapped) launch_group<true>(ctx, G, mem, A, B, C);
-    else launch_group<false>(ctx, G, mem, A, B, C);
+    if (!p.mapped) launch_group<kFused>(ctx, G, mem, A, B, C, parts);
+    else if (parts.c1 == 0) launch_group<kMapped>(ctx, G, mem, A, B, C, parts);
+    else launch_group<kParts>(ctx, G, mem, A, B, C, parts);
     MPSG_CUDA(cudaFreeAsync(mem, st));
   }
   if (ctx->debug_sync) {

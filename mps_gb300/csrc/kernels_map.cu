@@ -16,11 +16,12 @@ struct BlockRegs {
   int rs0, rs1, rs2, cs0, cs1, cs2;
 };
 
-__device__ __forceinline__ BlockRegs load_block(const MapBlock* b) {
+__device__ __forceinline__ BlockRegs load_block(const MapBlock* b, int64_t d1, int64_t d2 = 0,
+                                                int64_t d3 = 0) {
   const int4* p = reinterpret_cast<const int4*>(b);
   const int4 x = __ldg(p), y = __ldg(p + 1);
-  return BlockRegs{(int64_t)(((unsigned long long)(unsigned)x.y << 32) | (unsigned)x.x),
-                   x.z, x.w, y.x, y.y, y.z, y.w};
+  const int64_t base = (int64_t)(((unsigned long long)(unsigned)x.y << 32) | (unsigned)x.x);
+  return BlockRegs{part_base(base, d1, d2, d3), x.z, x.w, y.x, y.y, y.z, y.w};
 }
 
 __device__ __forceinline__ int64_t row_part(const BlockRegs& b, const int4& e) {
@@ -43,15 +44,16 @@ constexpr int kChunk = 128, kSmallRows = 32, kSmallCols = 4;
 
 // Offset of a row's (or column's) element at contracted index x, through its block table.
 __device__ __forceinline__ int64_t mapped_at(const MapBlock* __restrict__ tab, const int4& row,
-                                             const int4& x) {
-  const BlockRegs b = load_block(tab + (x.x & kComboMask));
+                                             const int4& x, int64_t d1) {
+  const BlockRegs b = load_block(tab + (x.x & kComboMask), d1);
   return row_part(b, row) + col_part(b, x);
 }
 
 __global__ void __launch_bounds__(kSmallRows * kSmallCols) contract_small_kernel(
     const SmallProblem* __restrict__ probs, int nprob, int ntiles,
     const AxisEntry* __restrict__ axes, const MapBlock* __restrict__ blocks,
-    const double* __restrict__ A, const double* __restrict__ B, double* __restrict__ C) {
+    const double* __restrict__ A, const double* __restrict__ B, double* __restrict__ C,
+    const PartOffsets parts) {
   __shared__ double as[kChunk * kSmallRows], bs[kChunk * kSmallCols];
   const int4* ax = reinterpret_cast<const int4*>(axes);
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
@@ -71,7 +73,8 @@ __global__ void __launch_bounds__(kSmallRows * kSmallCols) contract_small_kernel
     const MapBlock* ta = blocks + P.blkA + (me.x & kComboMask) * P.nkc;
     const MapBlock* tb = blocks + P.blkB + (nl.x & kComboMask) * P.nkc;
     const BlockRegs bc =
-        load_block(blocks + P.blkC + (me.x & kComboMask) * P.nnc + (ne.x & kComboMask));
+        load_block(blocks + P.blkC + (me.x & kComboMask) * P.nnc + (ne.x & kComboMask), parts.c1,
+                   parts.c2, parts.c3);
     double acc = 0.0;
     for (int c0 = 0; c0 == 0 || c0 < P.K; c0 += kChunk) {
       const int4* ke = ax + P.axK + c0;
@@ -81,12 +84,12 @@ __global__ void __launch_bounds__(kSmallRows * kSmallCols) contract_small_kernel
 #pragma unroll
       for (int u = 0; u < kB; ++u) {
         const int k = (t >> 2) + kSmallRows * u;
-        if (k < kn) ob[u] = mapped_at(tb, nl, __ldg(ke + k));
+        if (k < kn) ob[u] = mapped_at(tb, nl, __ldg(ke + k), parts.b);
       }
 #pragma unroll
       for (int u = 0; u < kA; ++u) {
         const int k = w + kSmallCols * u;
-        if (k < kn) oa[u] = mapped_at(ta, me, __ldg(ke + k));
+        if (k < kn) oa[u] = mapped_at(ta, me, __ldg(ke + k), parts.a);
       }
       if (tile == blockIdx.x && c0 == 0) cudaGridDependencySynchronize();
       double va[kA], vb[kB];
@@ -104,7 +107,7 @@ __global__ void __launch_bounds__(kSmallRows * kSmallCols) contract_small_kernel
 #pragma unroll
         for (int u = 0; u < kA; ++u) {
           const int k = kPart + w + kSmallCols * u;
-          if (k < kn) va[u] = __ldg(A + mapped_at(ta, me, __ldg(ke + k)));
+          if (k < kn) va[u] = __ldg(A + mapped_at(ta, me, __ldg(ke + k), parts.a));
         }
 #pragma unroll
         for (int u = 0; u < kA; ++u) {
@@ -237,7 +240,7 @@ template <int KMAX, int ROWS>
 __global__ void __launch_bounds__(256) contract_thin_kernel(
     const ThinUnit* __restrict__ units, int nunits, const ThinOffset* __restrict__ offs,
     const int64_t* __restrict__ vals, const double* __restrict__ A, const double* __restrict__ B,
-    double* __restrict__ C) {
+    double* __restrict__ C, const PartOffsets parts) {
   __shared__ ThinShared s;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   cudaTriggerProgrammaticLaunchCompletion();
@@ -246,10 +249,15 @@ __global__ void __launch_bounds__(256) contract_thin_kernel(
     const double* L = u.longB ? B : A;
     const double* S = u.longB ? A : B;
     __syncthreads();  // the previous unit has been read
-    if (threadIdx.x < u.K + u.T) s.o[threadIdx.x] = offs[u.offs + threadIdx.x];
+    if (threadIdx.x < u.K + u.T) {
+      ThinOffset o = offs[u.offs + threadIdx.x];
+      o.off = threadIdx.x < u.K ? part_base(o.off, u.longB ? parts.b : parts.a, 0, 0)
+                                : part_base(o.off, parts.c1, parts.c2, parts.c3);
+      s.o[threadIdx.x] = o;
+    }
     if (it == blockIdx.x) cudaGridDependencySynchronize();
     for (int x = threadIdx.x; x < u.T * u.K; x += blockDim.x)
-      s.b[x] = __ldg(S + __ldg(vals + u.vals + x));
+      s.b[x] = __ldg(S + part_base(__ldg(vals + u.vals + x), u.longB ? parts.a : parts.b, 0, 0));
     __syncthreads();
     if (threadIdx.x < u.T) {
       const double* b = s.b + threadIdx.x * u.K;
@@ -385,17 +393,23 @@ void plan_direct(const std::vector<MapProblem>& map, const std::vector<GemmTask>
 }
 
 bool DirectPlan::build(const ContractPlan& p, const TensorMeta& A, const TensorMeta& B,
-                       int num_sms, cudaStream_t st) {
-  const std::vector<MapProblem> map = build_contract_map(p, A, B);
+                       int num_sms, cudaStream_t st, bool ca, bool cb) {
+  std::vector<MapProblem> map = build_contract_map(p, A, B);
+  if (ca || cb) map = complex_map(map, ca, cb);
   if (map.empty()) return false;
+  std::vector<GemmTask> gemms = p.mm.gemms;  // (addresses come from the map)
+  for (GemmTask& g : gemms) {
+    if (ca) g.M *= 2;
+    if (cb) g.N *= 2;
+  }
   DirectTables t;
-  plan_direct(map, p.mm.gemms, num_sms, t);
+  plan_direct(map, gemms, num_sms, t);
   for (const auto& x : t.tiled)
     if (!f64tc::eligible(x.g)) return false;
   // nothing to save: the operands and the result are the fused matrices already
-  if (!t.tiled.empty() && p.fa.identity && p.fb.identity && p.split.identity) return false;
+  if (!ca && !cb && !t.tiled.empty() && p.fa.identity && p.fb.identity && p.split.identity) return false;
   stream = st;
-  flops = p.flops;
+  flops = p.flops * (ca ? 2 : 1) * (cb ? 2 : 1);
   for (const auto& x : t.tiled) tc_flops += 2.0 * x.g.M * x.g.N * x.g.K;
   TableImage img;
   const size_t os = img.add(t.small), ou = img.add(t.units), of = img.add(t.offs), ov = img.add(t.vals), oa = img.add(t.axes), ob = img.add(t.blocks);
@@ -421,15 +435,41 @@ DirectPlan::~DirectPlan() {
   if (d_tables) cudaFreeAsync(d_tables, stream);
 }
 
-bool launch_direct(Context* ctx, DirectPlan& p, const double* A, const double* B, double* C) {
+// (re, im) of a complex product from its four real ones, with the arithmetic of two linear combinations
+// in one pass and launch.
+__global__ void __launch_bounds__(256) complex_parts_kernel(int64_t n, double* __restrict__ rr,
+                                                            double* __restrict__ ri,
+                                                            const double* __restrict__ ir,
+                                                            const double* __restrict__ ii,
+                                                            double c_ri, double c_ir, double c_ii) {
+  cudaTriggerProgrammaticLaunchCompletion();
+  cudaGridDependencySynchronize();
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n;
+       e += (int64_t)gridDim.x * blockDim.x) {
+    rr[e] = fma(c_ii, ii[e], fma(1.0, rr[e], 0.0));
+    ri[e] = fma(c_ir, ir[e], fma(c_ri, ri[e], 0.0));
+  }
+}
+
+void launch_complex_parts(Context* ctx, int64_t n, double* rr, double* ri, const double* ir,
+                          const double* ii, double c_ri, double c_ir, double c_ii) {
+  if (n == 0) return;
+  const int64_t grid = std::min<int64_t>((n + 255) / 256, (int64_t)ctx->num_sms * 8);
+  launch_chained(complex_parts_kernel, dim3((unsigned)grid), dim3(256), 0, ctx->stream, 1, n, rr, ri,
+                 ir, ii, c_ri, c_ir, c_ii);
+  ctx->kernel_launches++;
+}
+
+bool launch_direct(Context* ctx, DirectPlan& p, const double* A, const double* B, double* C,
+                   const PartOffsets& parts) {
   cudaStream_t st = ctx->stream;
-  if (p.tc && !f64tc::launch(ctx, *p.tc, A, B, C)) return false;
+  if (p.tc && !f64tc::launch(ctx, *p.tc, A, B, C, parts)) return false;
   if (p.small_tiles || p.nunits) {
     KernelTimer timer(ctx, kKindGemmF64, p.flops - p.tc_flops);
     if (p.small_tiles) {
       const int grid = std::min(p.small_tiles, ctx->num_sms * 16);
       launch_chained(contract_small_kernel, dim3((unsigned)grid), dim3(kSmallRows * kSmallCols), 0, st,
-                     1, p.d_small, p.nsmall, p.small_tiles, p.d_axes, p.d_blocks, A, B, C);
+                     1, p.d_small, p.nsmall, p.small_tiles, p.d_axes, p.d_blocks, A, B, C, parts);
       ctx->kernel_launches++;
     }
     if (p.nunits) {
@@ -440,7 +480,7 @@ bool launch_direct(Context* ctx, DirectPlan& p, const double* A, const double* B
                                    : contract_thin_kernel<32, 1>;
       const int grid = std::min(p.nunits, ctx->num_sms * 8);
       launch_chained(kern, dim3((unsigned)grid), dim3(256), 0, st, 1, p.d_units, p.nunits, p.d_offs,
-                     p.d_vals, A, B, C);
+                     p.d_vals, A, B, C, parts);
       ctx->kernel_launches++;
     }
   }

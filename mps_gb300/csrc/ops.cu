@@ -305,13 +305,14 @@ static void ensure_fused(Context* ctx, DevContract& p) {
   p.fused = true;
 }
 
-static DirectPlan* direct_plan(Context* ctx, DevContract& p) {
-  if (!p.direct_tried) {
+static DirectPlan* direct_plan(Context* ctx, DevContract& p, bool ca = false, bool cb = false) {
+  const int i = (ca ? 1 : 0) + (cb ? 2 : 0);
+  if (!p.direct_tried[i]) {
     auto d = std::make_shared<DirectPlan>();
-    if (d->build(*p.host, p.metaA, p.metaB, ctx->num_sms, ctx->stream)) p.direct = d;
-    p.direct_tried = true;
+    if (d->build(*p.host, p.metaA, p.metaB, ctx->num_sms, ctx->stream, ca, cb)) p.direct[i] = d;
+    p.direct_tried[i] = true;
   }
-  return p.direct.get();
+  return p.direct[i].get();
 }
 
 std::shared_ptr<Buffer> contract_gemm(Context* ctx, DevContract& p, const DeviceTensor& a,
@@ -333,6 +334,47 @@ std::shared_ptr<Buffer> contract_gemm(Context* ctx, DevContract& p, const Device
   auto fc = alloc_buffer(ctx, p.host->mm.out.total);
   run_gemm(ctx, p.mm, pa, pb, fc->ptr, precision);
   return fc;
+}
+
+// The products of the parts of (ar + i ai)(br + i bi) in one set of launches: each operand is packed once
+// and the tiles of all products share one grid. Every product is rounded as in a contraction of its
+// own, then combined. A one-site H_eff on complex tensors, chi = 512: 392 us with four
+// contractions and two linear combinations per product, 127 us so.
+bool contract_complex(Context* ctx, const DeviceTensor& ar, const DeviceTensor* ai, double sa,
+                      const std::vector<int>& idxA, const DeviceTensor& br, const DeviceTensor* bi,
+                      double sb, const std::vector<int>& idxB, int precision, DeviceTensor& cr,
+                      DeviceTensor& ci) {
+  if (!ai && !bi) return false;
+  auto p = get_contract_plan(ctx, ar.meta, idxA, br.meta, idxB);
+  if (p->host->scalar) return false;
+  if (arithmetic(precision) != 0 && p->host->tiled_flops() > kSplitContractFlops) return false;
+  DirectPlan* d = direct_plan(ctx, *p, ai != nullptr, bi != nullptr);
+  if (!d) return false;
+  DeviceTensor part[4];
+  const int np = ai && bi ? 4 : 2;
+  for (int i = 0; i < np; ++i) {
+    part[i].ctx = ctx;
+    part[i].meta = p->host->split.out;
+    part[i].buf = alloc_buffer(ctx, part[i].meta.total);
+  }
+  PartOffsets o;
+  if (ai) o.a = ai->data() - ar.data();
+  if (bi) o.b = bi->data() - br.data();
+  o.c1 = part[1].data() - part[0].data();
+  if (np == 4) {
+    o.c2 = part[2].data() - part[0].data();
+    o.c3 = part[3].data() - part[0].data();
+  }
+  if (!launch_direct(ctx, *d, ar.data(), br.data(), part[0].data(), o)) return false;
+  const int64_t n = part[0].meta.total;
+  if (np == 4)
+    launch_complex_parts(ctx, n, part[0].data(), part[1].data(), part[2].data(), part[3].data(), sb,
+                         sa, -sa * sb);
+  else if ((ai ? sa : sb) != 1.0)
+    launch_lincomb(ctx, n, {part[1].data()}, {ai ? sa : sb}, part[1].data());
+  cr = std::move(part[0]);
+  ci = std::move(part[1]);
+  return true;
 }
 
 DeviceTensor contract(Context* ctx, const DeviceTensor& a, const std::vector<int>& idxA,

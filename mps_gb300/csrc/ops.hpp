@@ -33,6 +33,12 @@ std::shared_ptr<DevContract> get_contract_plan(Context* ctx, const TensorMeta& A
                                                const TensorMeta& B,
                                                const std::vector<int>& idxB);
 // Returns an empty tensor (no buffer, no legs) and sets *scalar when every leg is contracted.
+// (ar + i sa ai)(br + i sb bi), either imaginary part null; false where the parts have to be contracted
+// one by one (two real operands, a full contraction, slices, no index map or no scratch).
+bool contract_complex(Context* ctx, const DeviceTensor& ar, const DeviceTensor* ai, double sa,
+                      const std::vector<int>& idxA, const DeviceTensor& br, const DeviceTensor* bi,
+                      double sb, const std::vector<int>& idxB, int precision, DeviceTensor& cr,
+                      DeviceTensor& ci);
 DeviceTensor contract(Context* ctx, const DeviceTensor& a, const std::vector<int>& idxA,
                       const DeviceTensor& b, const std::vector<int>& idxB, int precision,
                       double* scalar);

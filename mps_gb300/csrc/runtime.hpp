@@ -150,8 +150,9 @@ struct DevContract {
   DevCopyPlan fa, fb, split;
   DevGemmPlan mm;
   bool fused = false;                  // fa, fb, split and mm are on the device
-  bool direct_tried = false;
-  std::shared_ptr<DirectPlan> direct;  // FP64 without fused copies (null: not for this structure)
+  // FP64 without fused copies (null: not for this structure), by [A complex] + 2 [B complex]
+  bool direct_tried[4] = {false, false, false, false};
+  std::shared_ptr<DirectPlan> direct[4];
   size_t device_bytes() const { return mm.device_bytes(); }
   ~DevContract();
 };
