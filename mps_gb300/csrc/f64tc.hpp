@@ -17,7 +17,7 @@ constexpr int64_t kMaxK = 65536;           // whole K summed in 64 bits (fits up
 
 // One sector GEMM as the kernels see it: R is the operand on the 128-row side, S the one on the
 // 80-row side. Either operand of the contraction may be R (swap: it is B, and the output is written
-// transposed), whichever pads fewer tiles. Elements are found by strides (fused matrices) or, in a
+// transposed), see plan_group. Elements are found by strides (fused matrices) or, in a
 // mapped group, by axis entries and block tables (the tensors themselves).
 struct Problem {
   int64_t M, N, K;            // rows of R, rows of S, contracted
