@@ -32,8 +32,8 @@ struct Problem {
   int32_t fastA, fastB;       // rows (1) or k (0) contiguous in memory
 };
 
-// One output tile, or one of `parts` pieces of its K steps: the pieces leave their sums in scratch
-// slots slot .. slot + parts - 1 and the last one to arrive adds them up and writes the tile.
+// One output tile, or one of `parts` pieces of its K steps: the pieces add their sums to scratch slot
+// `slot` and the last one to arrive writes the tile.
 struct Tile {
   int32_t prob, mi, ni, ks0, ks1;  // K steps [ks0, ks1)
   int32_t slot, part, parts;

@@ -288,6 +288,8 @@ struct MapCursor {
 template <Access MAP>
 using Cursor = std::conditional_t<MAP == kFused, FusedCursor, MapCursor<MAP == kParts>>;
 
+constexpr int64_t kSlotWords = (int64_t)BM * BN * 2;  // 64-bit words of a cut tile's sums
+
 // One cluster per item (32 rows of one operand, whole K), its K steps shared out over the CTAs: each
 // CTA keeps its part in shared memory while it finds the rows' largest elements, the CTAs exchange
 // those, and the digits are cut from the kept part. HBM and L2 see 8 bytes read and 14 written
@@ -301,7 +303,7 @@ __global__ void __launch_bounds__(256) pack_f64_kernel(
     const AxisEntry* __restrict__ axes, const MapBlock* __restrict__ blocks,
     const double* __restrict__ A, const double* __restrict__ B, int32_t* __restrict__ RA,
     int32_t* __restrict__ RB, __nv_bfloat16* __restrict__ packA, __nv_bfloat16* __restrict__ packB,
-    int64_t rowsA, int64_t rowsB, int* __restrict__ arrivals, int nslots, int64_t partA,
+    int64_t rowsA, int64_t rowsB, int* __restrict__ arrivals, ulonglong2* __restrict__ slots, int nslots, int64_t partA,
     int64_t partB) {
   extern __shared__ double xs[];  // [k][row], rows padded to kPadRows
   __shared__ uint32_t red[8][33], rlow[8][33];  // largest high words, all low words or-ed
@@ -328,8 +330,12 @@ __global__ void __launch_bounds__(256) pack_f64_kernel(
   const int64_t kb = (int64_t)s0 * BK, ke = min((int64_t)s1 * BK, K);
   const bool keep = per <= cache_steps;
   cudaGridDependencySynchronize();
-  if (blockIdx.x == 0)  // the GEMM's arrival counters
+  // the GEMM's arrival counters and the sums of its cut tiles
+  if (blockIdx.x == 0)
     for (int i = t; i < nslots; i += blockDim.x) arrivals[i] = 0;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + t; i < nslots * (kSlotWords / 2);
+       i += (int64_t)gridDim.x * blockDim.x)
+    slots[i] = make_ulonglong2(0, 0);
   // largest |x| of each row's part: lanes along whichever axis is contiguous
   if (side ? P.fastB : P.fastA) {
     uint32_t m = 0, lo = 0;
@@ -491,7 +497,6 @@ __device__ __noinline__ void fma_chains(const Problem& P, int64_t row, int64_t n
   }
 }
 
-constexpr int64_t kSlotLo = (int64_t)BM * BN * 8, kSlotBytes = (int64_t)BM * BN * 12;
 
 // Persistent, one CTA per SM: warp 0 TMA producer, warp 1 TMEM allocator and MMA issuer, 20
 // epilogue warps (five per TMEM lane quarter, 16 columns each). Every mbarrier wait is bounded;
@@ -504,7 +509,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f64tc_kernel(
     const int32_t* __restrict__ RA, const int32_t* __restrict__ RB,
     const AxisEntry* __restrict__ axes, const MapBlock* __restrict__ blocks,
     const double* __restrict__ A, const double* __restrict__ B, double* __restrict__ C,
-    unsigned char* __restrict__ slots, int* __restrict__ arrivals, int* __restrict__ err,
+    unsigned long long* __restrict__ slots, int* __restrict__ arrivals, int* __restrict__ err,
     const __grid_constant__ PartOffsets parts) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = (uint8_t*)(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
@@ -666,17 +671,23 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f64tc_kernel(
         }
       }
       if (!ok) break;
+      const int64_t row = (int64_t)tr.mi * BM + lrow, n0 = (int64_t)tr.ni * BN + col0;
+      const int nc = (int)min((int64_t)kEpiCols, P.N - n0);
       if (tr.parts > 1) {
-        // element (row, column) of part q at (column * BM + row) of slot q
-        const int64_t at = (int64_t)col0 * BM + lrow;
-        unsigned char* mine = slots + (int64_t)(tr.slot + tr.part) * kSlotBytes;
+        // element (row, column) at column * BM + row of the tile's slot: the 64-bit sums, then the small
+        // ones in units of 2^-60 (integers both, so their order does not matter)
+        unsigned long long* s = slots + tr.slot * kSlotWords + col0 * BM + lrow;
+        if (row < P.M) {
 #pragma unroll
-        for (int j = 0; j < kEpiCols; ++j) {
-          reinterpret_cast<long long*>(mine)[at + j * BM] = hi[j];
-          reinterpret_cast<float*>(mine + kSlotLo)[at + j * BM] = lo[j];
+          for (int j = 0; j < kEpiCols; ++j)
+            if (j < nc) {
+              atomicAdd(s + j * BM, (unsigned long long)hi[j]);
+              atomicAdd(s + BM * BN + j * BM,
+                        (unsigned long long)__float2ll_rn(lo[j] * __uint_as_float((127u + 60u) << 23)));
+            }
         }
         __threadfence();
-        mbar_arrive(esync);  // every thread's sums are in the slot
+        mbar_arrive(esync);  // every thread's sums are on their way before the arrival counts
         if (!mbar_wait(esync, 0, abort_flag, err, 6)) break;
         if (threadIdx.x == 64) {
           __threadfence();
@@ -686,27 +697,16 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f64tc_kernel(
         if (!mbar_wait(esync, 1, abort_flag, err, 6)) break;
         if (!*last_part) continue;
         __threadfence();
-        // integer sums do not depend on the order; the FP32 ones are taken part by part
-        float own[kEpiCols];
-#pragma unroll
-        for (int j = 0; j < kEpiCols; ++j) {
-          own[j] = lo[j];
-          lo[j] = 0.f;
-        }
-        for (int q = 0; q < tr.parts; ++q) {
-          const unsigned char* s = slots + (int64_t)(tr.slot + q) * kSlotBytes;
+        if (row < P.M) {
 #pragma unroll
           for (int j = 0; j < kEpiCols; ++j) {
-            if (q != tr.part) hi[j] += __ldcg(reinterpret_cast<const long long*>(s) + at + j * BM);
-            lo[j] += q != tr.part ? __ldcg(reinterpret_cast<const float*>(s + kSlotLo) + at + j * BM)
-                                  : own[j];
+            hi[j] = j < nc ? (long long)__ldcg(s + j * BM) : 0;
+            const long long l = j < nc ? (long long)__ldcg(s + BM * BN + j * BM) : 0;
+            lo[j] = (float)l * __uint_as_float((127u - 60u) << 23);
           }
         }
       }
-      const int64_t row = (int64_t)tr.mi * BM + lrow;
       if (row < P.M) {
-        const int64_t n0 = (int64_t)tr.ni * BN + col0;
-        const int nc = (int)min((int64_t)kEpiCols, P.N - n0);
         const int er = K ? RA[P.rA + row] : kRowZero;
         const int32_t* RBp = RB + P.rB + n0;
         bool bad = er == kRowBad;
@@ -743,7 +743,8 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f64tc_kernel(
 
 constexpr size_t kGroupBytes = size_t(2) << 30;  // packed operands per launch pair
 constexpr int kMinPart = 3, kMaxParts = 16;      // K steps of a piece of a tile, pieces
-constexpr double kCutSteps = 1.5, kTileSteps = 1.0;
+// (with 1.5 for kCutSteps chi = 2048 takes 562 us instead of 549, chi = 517 the same)
+constexpr double kCutSteps = 2.5, kTileSteps = 1.0;
 
 int64_t ceil_div(int64_t a, int64_t b) { return (a + b - 1) / b; }
 
@@ -763,7 +764,7 @@ bool eligible(const GemmTask& t) { return t.K <= kMaxK; }
 size_t Group::scratch_bytes() const {
   return round256((size_t)rowsA * BK * 2 * kSlices) + round256((size_t)rowsB * BK * 2 * kSlices) +
          round256(sizeof(int32_t) * (size_t)rA) + round256(sizeof(int32_t) * (size_t)rB) +
-         round256(sizeof(int) * (size_t)nslots) + (size_t)nslots * kSlotBytes;
+         round256(sizeof(int) * (size_t)nslots) + (size_t)nslots * kSlotWords * 8;
 }
 
 // Whether the rows of an operand table, rather than k, run along the unit stride of its blocks
@@ -875,9 +876,9 @@ void plan_group(const std::vector<Task>& g, int num_sms, Group& G, GroupTables& 
     t.probs.push_back(P);
   }
   // Tiles of very different K, or fewer tiles than SMs, leave SMs idle: then tiles are cut along K
-  // into pieces of at most `most` K steps. A piece costs its sums' way through L2 (120 KB written
-  // and read, about kCutSteps K steps), a tile its first loads and its stores (kTileSteps); the
-  // limit with the shortest estimated busiest SM is taken, the uncut list first.
+  // into pieces of at most `most` K steps, which add their sums up in L2. A piece costs that (160 KB,
+  // and for the last one its way back; about kCutSteps K steps), a tile its first loads and its stores
+  // (kTileSteps); the limit with the shortest estimated busiest SM is taken, the uncut list first.
   auto cut_at = [&](int most, std::vector<Tile>& cut, int64_t& slots) {
     cut.clear();
     slots = 0;
@@ -892,7 +893,7 @@ void plan_group(const std::vector<Task>& g, int num_sms, Group& G, GroupTables& 
         y.parts = parts;
         cut.push_back(y);
       }
-      if (parts > 1) slots += parts;
+      if (parts > 1) ++slots;
     }
     std::stable_sort(cut.begin(), cut.end(), [](const Tile& a, const Tile& b) {
       return a.ks1 - a.ks0 > b.ks1 - b.ks0;
@@ -992,7 +993,8 @@ static void launch_group(Context* ctx, Group& G, unsigned char* mem, const doubl
   int32_t* RA = (int32_t*)(mem + bA + bB);
   int32_t* RB = (int32_t*)(mem + bA + bB + round256(sizeof(int32_t) * (size_t)G.rA));
   int* arrivals = (int*)((unsigned char*)RB + round256(sizeof(int32_t) * (size_t)G.rB));
-  unsigned char* slots = (unsigned char*)arrivals + round256(sizeof(int) * (size_t)G.nslots);
+  unsigned long long* slots =
+      (unsigned long long*)((unsigned char*)arrivals + round256(sizeof(int) * (size_t)G.nslots));
   CUtensorMap tmA, tmB;
   make_slice_map(&tmA, packA, G.rowsA, kSlices, BM, BK, BK);
   make_slice_map(&tmB, packB, G.rowsB, kSlices, BN, BK, BK);
@@ -1008,7 +1010,8 @@ static void launch_group(Context* ctx, Group& G, unsigned char* mem, const doubl
                         kCacheSteps * BK * kPadRows * (int)sizeof(double));
     launch_chained(pack_f64_kernel<MAP>, dim3((unsigned)G.nitems * (unsigned)ncta), dim3(256),
                    (size_t)smem, st, ncta, G.d_probs, G.d_items, ncta, steps, G.d_axes, G.d_blocks,
-                   A, B, RA, RB, packA, packB, G.rowsA, G.rowsB, arrivals, (int)G.nslots, parts.a,
+                   A, B, RA, RB, packA, packB, G.rowsA, G.rowsB, arrivals, (ulonglong2*)slots,
+                   (int)G.nslots, parts.a,
                    parts.b);
     ctx->kernel_launches++;
   }
