@@ -433,10 +433,25 @@ static const std::vector<int> kH2A = {1, -1, -2, 4, 5}, kH2B = {-1, 2, 3, -2};
 static const std::vector<int> kH3A = {1, 2, -1, -2, 5}, kH3B = {-1, 3, 4, -2};
 static const std::vector<int> kH4A = {1, 2, 3, -1, -2}, kH4B = {-2, -1, 4};
 
+// The arithmetic of a two-site H_eff. Five slices pay from about 4 GFLOP on, where the MMAs that they save
+// outweigh their extra passes (fused copies, exponents, W folded into the environments): FP64 / 5
+// slices in us, chi = 48 17 / 101, 517 106 / 172, 1024 194 / 254, 1448 330 / 334, 2048 549 / 466.
+// Smaller operators asked for with five slices get FP64 results. (Fewer slices are kept at every
+// size: a batch runs slices, and its operators agree with single ones to rounding there.)
+constexpr double kHeffFp64Flops = 4e9;
+
+static int heff_arithmetic(Context* ctx, int precision, const TensorMeta& v, const TensorMeta& envL,
+                           const TensorMeta& envR, const TensorMeta& W1, const TensorMeta& W2) {
+  precision = arithmetic(precision);
+  return precision == 5 && applymps2site_flops(ctx, v, envL, envR, W1, W2) <= kHeffFp64Flops
+             ? 0
+             : precision;
+}
+
 DeviceTensor applymps2site(Context* ctx, const DeviceTensor& v, const DeviceTensor& envL,
                            const DeviceTensor& envR, const DeviceTensor& W1,
                            const DeviceTensor& W2, int precision) {
-  precision = arithmetic(precision);
+  precision = heff_arithmetic(ctx, precision, v.meta, envL.meta, envR.meta, W1.meta, W2.meta);
   if (precision != 0) {  // split-precision path: prepared (W-folded) operator, built per call here
     auto op = heff_create(ctx, v.meta, envL, envR, W1, W2, precision);
     return heff_apply(*op, v);
@@ -505,7 +520,7 @@ DeviceTensor applymps2site_host(Context* ctx, const DeviceTensor& v, const Devic
   }
   MPSG_CUDA(cudaEventRecord(ctx->copy_ev[2], cs));  // v
   DeviceTensor out;
-  if (arithmetic(precision) != 0) {
+  if (heff_arithmetic(ctx, precision, v.meta, envL.meta, envR.meta, W1.meta, W2.meta) != 0) {
     auto op = heff_create(ctx, v.meta, envL, envR, W1, W2, precision, ctx->copy_ev[0],
                           ctx->copy_ev[1]);
     MPSG_CUDA(cudaStreamWaitEvent(ctx->stream, ctx->copy_ev[2], 0));
@@ -702,7 +717,7 @@ std::shared_ptr<HeffOp> heff_create(Context* ctx, const TensorMeta& vmeta, const
   op->ctx = ctx;
   op->vmeta = vmeta;
   op->ref_flops = applymps2site_flops(ctx, vmeta, envL.meta, envR.meta, W1.meta, W2.meta);
-  op->precision = arithmetic(precision);
+  op->precision = heff_arithmetic(ctx, precision, vmeta, envL.meta, envR.meta, W1.meta, W2.meta);
   if (op->precision == 0) {
     // precision 0 reads the tensors at every application; a slice count takes them as they are now
     const bool keep = precision != 0;

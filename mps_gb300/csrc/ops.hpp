@@ -6,8 +6,8 @@
 
 namespace mpsg {
 
-// Slice counts from this one on run as FP64 (see arithmetic() in ops.cu); batched operators keep their
-// split-precision slices.
+// Slice counts from this one on run as FP64, and five slices for small operators (see arithmetic() and
+// heff_arithmetic() in ops.cu); batched operators keep their split-precision slices.
 constexpr int kFp64Slices = 6;
 
 void context_init(Context* ctx, int device);
@@ -32,13 +32,13 @@ std::shared_ptr<DevContract> get_contract_plan(Context* ctx, const TensorMeta& A
                                                const std::vector<int>& idxA,
                                                const TensorMeta& B,
                                                const std::vector<int>& idxB);
-// Returns an empty tensor (no buffer, no legs) and sets *scalar when every leg is contracted.
 // (ar + i sa ai)(br + i sb bi), either imaginary part null; false where the parts have to be contracted
 // one by one (two real operands, a full contraction, slices, no index map or no scratch).
 bool contract_complex(Context* ctx, const DeviceTensor& ar, const DeviceTensor* ai, double sa,
                       const std::vector<int>& idxA, const DeviceTensor& br, const DeviceTensor* bi,
                       double sb, const std::vector<int>& idxB, int precision, DeviceTensor& cr,
                       DeviceTensor& ci);
+// Returns an empty tensor (no buffer, no legs) and sets *scalar when every leg is contracted.
 DeviceTensor contract(Context* ctx, const DeviceTensor& a, const std::vector<int>& idxA,
                       const DeviceTensor& b, const std::vector<int>& idxB, int precision,
                       double* scalar);
