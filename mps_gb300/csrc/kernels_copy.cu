@@ -380,6 +380,8 @@ __global__ void __launch_bounds__(32 * kBulkWarps, 2) copy_rows_bulk_kernel(
     const BulkRow* __restrict__ rows, int64_t nrows, const double* __restrict__ src,
     double* __restrict__ dst, int* __restrict__ err) {
   extern __shared__ __align__(128) unsigned char bulk_smem[];
+  cudaTriggerProgrammaticLaunchCompletion();
+  cudaGridDependencySynchronize();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   unsigned char* slots = bulk_smem + (size_t)warp * kBulkStages * kSlotBytes;
   uint64_t* bars = reinterpret_cast<uint64_t*>(bulk_smem + (size_t)kBulkWarps * kBulkStages *
@@ -638,9 +640,8 @@ void launch_copy(Context* ctx, const DevCopyPlan& p, const double* src, double* 
     const int64_t ctas = (p.nrows + kBulkWarps - 1) / kBulkWarps;
     const int64_t grid = std::min<int64_t>(ctas, (int64_t)ctx->num_sms * 2);
     KernelTimer timer(ctx, kKindCopy);
-    copy_rows_bulk_kernel<<<(unsigned)grid, 32 * kBulkWarps, kBulkSmem, ctx->stream>>>(
-        p.d_rows, p.nrows, src, dst, ctx->d_copy_err);
-    MPSG_CUDA(cudaGetLastError());
+    launch_chained(copy_rows_bulk_kernel, dim3((unsigned)grid), dim3(32 * kBulkWarps),
+                   (size_t)kBulkSmem, ctx->stream, 1, p.d_rows, p.nrows, src, dst, ctx->d_copy_err);
     ctx->kernel_launches++;
   }
   if (p.ntiles > 0) {

@@ -194,6 +194,8 @@ __global__ void __launch_bounds__(256) pack_exponents_kernel(
   __shared__ unsigned long long red[8][33];
   const int t = threadIdx.x;
   const int rb = is_b ? kExpRowsB : kExpRowsA;
+  cudaTriggerProgrammaticLaunchCompletion();
+  cudaGridDependencySynchronize();
   for (int64_t it = blockIdx.x; it < nitems; it += gridDim.x) {
     const int p = find_problem(item_prefix, nprob, it);
     const Problem P = probs[p];
@@ -267,6 +269,8 @@ __global__ void __launch_bounds__(256) pack_slices_kernel(
     const double* __restrict__ X, const int16_t* __restrict__ E, const int32_t* __restrict__ R,
     __nv_bfloat16* __restrict__ out) {
   constexpr int kBeta = kSliceBits;
+  cudaTriggerProgrammaticLaunchCompletion();
+  cudaGridDependencySynchronize();
   for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x) {
     const int p = find_problem(tile_prefix, nprob, t);
     const Problem P = probs[p];
@@ -441,6 +445,8 @@ __global__ void __launch_bounds__(kExactThreads, 1) split_gemm_kernel(
     fence_barrier_init();
   }
   if (warp == 1) tmem_alloc(tmem_slot, CF::kTmemCols);
+  cudaTriggerProgrammaticLaunchCompletion();
+  cudaGridDependencySynchronize();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -689,6 +695,8 @@ __global__ void __launch_bounds__(192, 1) split_gemm_fast_kernel(
     fence_barrier_init();
   }
   if (warp == 1) tmem_alloc(tmem_slot, CF::kTmemCols);
+  cudaTriggerProgrammaticLaunchCompletion();
+  cudaGridDependencySynchronize();
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -1039,8 +1047,9 @@ static void launch_gemm_t(Context* ctx, SplitPlan& sp, double* C) {
     split_gemm_fast_kernel<S <= 3 ? S : 3><<<grid, 192, FCF::kSmemBytes, ctx->stream>>>(
         sp.tmA, sp.tmB, sp.d_probs, sp.d_tiles, sp.ntiles, sp.d_RA, sp.d_CB, C, sp.d_err);
   } else {
-    split_gemm_kernel<S, BN><<<grid, CF::kThreads, CF::kSmemBytes, ctx->stream>>>(
-        sp.tmA, sp.tmB, sp.d_probs, sp.d_tiles, sp.ntiles, sp.d_RA, sp.d_CB, C, sp.d_err);
+    launch_chained(split_gemm_kernel<S, BN>, dim3((unsigned)grid), dim3(CF::kThreads),
+                   (size_t)CF::kSmemBytes, ctx->stream, 1, sp.tmA, sp.tmB, sp.d_probs, sp.d_tiles,
+                   sp.ntiles, sp.d_RA, sp.d_CB, C, sp.d_err);
   }
   MPSG_CUDA(cudaGetLastError());
 }
@@ -1061,22 +1070,18 @@ static void launch_t(Context* ctx, SplitPlan& sp, const double* A, const double*
                                 ctx->stream));
       KernelTimer timer(ctx, kKindPack);
       int g = (int)std::min<int64_t>(nitems, (int64_t)ctx->num_sms * 8);
-      pack_exponents_kernel<<<g, 256, 0, ctx->stream>>>(
-          sp.d_probs, side ? sp.d_rowB_prefix : sp.d_rowA_prefix, sp.nprob, nitems, side, sp.seg,
-          sp.fast ? 0 : 1,
-          X, E, R);
-      MPSG_CUDA(cudaGetLastError());
+      launch_chained(pack_exponents_kernel, dim3((unsigned)g), dim3(256), 0, ctx->stream, 1, sp.d_probs,
+                     side ? sp.d_rowB_prefix : sp.d_rowA_prefix, sp.nprob, nitems, side, sp.seg,
+                     sp.fast ? 0 : 1, X, E, R);
       ctx->kernel_launches++;
     }
     if (ntile) {
       KernelTimer timer(ctx, kKindPackSlices);
       int g = (int)std::min<int64_t>(ntile, (int64_t)ctx->num_sms * 8);
-      pack_slices_kernel<S><<<g, 256, 0, ctx->stream>>>(
-          sp.d_probs, side ? sp.d_packB_prefix : sp.d_packA_prefix, sp.nprob, ntile, side, chunk,
-          sp.fast ? 1 : 0,
-          side ? sp.bn : BM, side ? sp.rowsB : sp.rowsA, X, E, R,
-          (__nv_bfloat16*)(side ? sp.d_packB : sp.d_packA));
-      MPSG_CUDA(cudaGetLastError());
+      launch_chained(pack_slices_kernel<S>, dim3((unsigned)g), dim3(256), 0, ctx->stream, 1, sp.d_probs,
+                     side ? sp.d_packB_prefix : sp.d_packA_prefix, sp.nprob, ntile, side, chunk,
+                     sp.fast ? 1 : 0, side ? sp.bn : BM, side ? sp.rowsB : sp.rowsA, X, E, R,
+                     (__nv_bfloat16*)(side ? sp.d_packB : sp.d_packA));
       ctx->kernel_launches++;
     }
   }
