@@ -5,6 +5,8 @@
 // Measured, ground-state solve at chi = 256 (19 products, krylovdim 5, 8 cycles): 4.6 ms with a dozen
 // launches and one host synchronisation per step and the projected matrix decomposed by one warp
 // (112 us a cycle), 2.6 ms with one launch per step (21 us) and one synchronisation per cycle.
+#include <cooperative_groups.h>
+
 #include <algorithm>
 #include <cmath>
 #include <cstring>
@@ -61,6 +63,12 @@ constexpr int kMaxKrylov = 32;
 constexpr int kVecThreads = 256;
 constexpr long long kBarrierCycles = 4000000000LL;  // about 2 s at the maximum SM clock
 
+// Short vectors are left to one cluster of so many blocks, which meets at its hardware barrier (0.4 us
+// against about 2 us at a counter) and takes up to kClusterRows elements per thread: from about there
+// on, the FP64 pipes of more SMs save more than the barriers cost. chi = 64 DMRG sweep of 32 sites
+// 91.0 ms at the counter, 88.1 ms so.
+constexpr int kClusterBlocks = 8, kClusterRows = 3;
+
 // The vector part of a Lanczos solve runs as cooperative launches whose blocks meet at a counter in
 // device memory: one launch per Krylov step instead of a dozen (dots, sums, coefficients,
 // updates, twice, then the norm and the scaling), each of which would read the vectors again and
@@ -75,6 +83,10 @@ struct GridBarrier {
 __device__ __forceinline__ void grid_barrier(const GridBarrier& b, int i) {
   if (gridDim.x == 1) {
     __syncthreads();
+    return;
+  }
+  if (b.count == nullptr) {  // the grid is one cluster
+    cooperative_groups::this_cluster().sync();
     return;
   }
   __threadfence();
@@ -93,18 +105,29 @@ __device__ __forceinline__ void grid_barrier(const GridBarrier& b, int i) {
   __syncthreads();
 }
 
-// Sum of every thread's v[0..n) over the block into part[j * gridDim.x + blockIdx.x].
+// Sum of every thread's v[0..n) over the block into part[j * gridDim.x + blockIdx.x] (v is used up). The
+// lanes halve the list as they go: N / 2 additions, N / 4, .., one a step, instead of five per value.
 template <int N>
-__device__ __forceinline__ void block_partials(const double (&v)[N], int n, double* part) {
+__device__ __forceinline__ void block_partials(double (&v)[N], int n, double* part) {
   __shared__ double sh[kVecThreads / 32][N];
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  int j0 = 0;  // the value this lane holds a part of
 #pragma unroll
-  for (int j = 0; j < N; ++j) {
-    if (j >= n) break;
-    double x = v[j];
-    for (int o = 16; o; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    if (lane == 0) sh[w][j] = x;
+  for (int o = 16, m = N / 2; o; o >>= 1, m >>= 1) {
+    if (m == 0) {
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+      continue;
+    }
+    const bool upper = (lane & o) != 0;
+    if (upper) j0 += m;
+#pragma unroll
+    for (int j = 0; j < m; ++j) {
+      const double keep = upper ? v[j + m] : v[j], give = upper ? v[j] : v[j + m];
+      v[j] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+    }
   }
+  constexpr int kSame = N >= 32 ? 1 : 32 / N;  // lanes that hold one value
+  if ((lane & (kSame - 1)) == 0) sh[w][j0] = v[0];
   __syncthreads();
   for (int j = threadIdx.x; j < n; j += blockDim.x) {
     double x = 0.0;
@@ -263,11 +286,28 @@ __global__ void __launch_bounds__(kVecThreads) krylov_restart_kernel(
   }
 }
 
+template <class Args>
+void launch_clustered(void (*kernel)(Args), dim3 grid, dim3 block, cudaStream_t st, int cluster,
+                      const Args& a) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)cluster;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  MPSG_CUDA(cudaLaunchKernelEx(&cfg, kernel, a));
+}
+
 // Device scratch and launches of one solve.
 struct LanczosWork {
   Context* ctx;
   int kd, grid;
   int64_t n;
+  bool cluster;
   unsigned barriers = 0;
   std::shared_ptr<Buffer> buf;
   double *part, *out;     // partial sums; per step of a cycle (alpha, beta), then the start norm
@@ -278,6 +318,8 @@ struct LanczosWork {
     // by the FP64 pipes of the SMs that take part (22 FMAs per element at K = 5), so they spread
     grid = (int)std::max<int64_t>(
         1, std::min<int64_t>(ctx->num_sms, (n + kVecThreads - 1) / kVecThreads));
+    cluster = n <= (int64_t)kClusterBlocks * kClusterRows * kVecThreads;
+    if (cluster) grid = std::min(grid, kClusterBlocks);
     const int64_t np = 3 * (int64_t)kd * grid;
     buf = alloc_buffer(ctx, np + 2 * kd + 4);
     part = buf->ptr;
@@ -287,16 +329,20 @@ struct LanczosWork {
     MPSG_CUDA(cudaMemsetAsync(count, 0, 2 * sizeof(double), ctx->stream));
   }
   GridBarrier barrier(int n_barriers) {
-    GridBarrier b{count, (barriers + 1) * (unsigned)grid, err};
+    GridBarrier b{cluster ? nullptr : count, (barriers + 1) * (unsigned)grid, err};
     barriers += (unsigned)n_barriers;
     return b;
   }
   template <class Args>
   void run(void (*kernel)(Args), Args& a) {
+    ctx->kernel_launches++;
+    if (cluster) {
+      launch_clustered(kernel, dim3((unsigned)grid), dim3(kVecThreads), ctx->stream, grid, a);
+      return;
+    }
     void* p[] = {&a};
     MPSG_CUDA(cudaLaunchCooperativeKernel((const void*)kernel, dim3(grid), dim3(kVecThreads), p, 0,
                                           ctx->stream));
-    ctx->kernel_launches++;
   }
   // Krylov step number i of the cycle: w against V[0..K), next <- the rest normalised
   void step(int i, const std::vector<DeviceTensor>& V, int K, DeviceTensor& w, DeviceTensor& next) {
