@@ -38,8 +38,9 @@
 // Measured: one 4096 x 4000 x 4096 product 2.72 ms (49 TFLOP/s of FP64 work, 74% of the bf16 rate in
 // digit products; the FP64 pipe takes 125 ms). Before the MMAs were issued from code that the
 // whole warp runs in step (elect_one) 3.72 ms: 80 cycles per MMA went into moving its operands to
-// uniform registers. The two GEMMs of a two-site H_eff, packing + this kernel: chi = 2048 137 + 346 us
-// (FP64 pipe 9205), chi = 517 26 + 58 us (870). Relative error of N(0,1) products against extended
+// uniform registers. The two GEMMs of a two-site H_eff, packing + this kernel: chi = 2048 141 + 323 us
+// (FP64 pipe 9205; tensor cycles 42 and 53%, the epilogue's integer sums and stores of a tile, 13000
+// cycles, hold the next one's MMAs up). Relative error of N(0,1) products against extended
 // precision: 2e-16 (K = 33) to 1.4e-15 (K = 2050) on the FP64 pipe, 5e-17 here.
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
