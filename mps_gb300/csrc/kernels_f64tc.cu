@@ -295,8 +295,8 @@ constexpr int64_t kSlotWords = (int64_t)BM * BN * 2;  // 64-bit words of a cut t
 // CTA keeps its part in shared memory while it finds the rows' largest elements, the CTAs exchange
 // those, and the digits are cut from the kept part. HBM and L2 see 8 bytes read and 14 written
 // per element; about 60 integer and FP32 instructions. A part longer than kCacheSteps (K above
-// 8 x 256) is read again instead of kept.
-constexpr int kCacheSteps = 8, kPadRows = kRowBlock + 1, kMaxCluster = 8;
+// 8 x 192) is read again instead of kept: four CTAs fit an SM so, three with eight steps.
+constexpr int kCacheSteps = 6, kPadRows = kRowBlock + 1, kMaxCluster = 8;
 
 template <Access MAP>
 __global__ void __launch_bounds__(256) pack_f64_kernel(
@@ -1002,9 +1002,16 @@ static void launch_group(Context* ctx, Group& G, unsigned char* mem, const doubl
   set_smem_limit_once(ctx, smem_set, gemm_f64tc_kernel<MAP>, kSmemBytes);
   if (G.nitems) {
     KernelTimer timer(ctx, kKindPack);
-    // CTAs per item: as many as keep an item's part in shared memory
+    // CTAs per item: as many as keep an item's part in shared memory, and more while that fills the chip
+    // (up to eight CTAs per SM, a CTA's barriers and latencies being most of its time; two K steps
+    // each are worth one). Two-site H_eff, one CTA per eight steps / so: chi = 517 106 / 98 us, 2048
+    // 550 / 536; complex one-site product 122 / 111 us. With four steps as the limit, or more CTAs
+    // than that, chi = 2048 and 1024 lose what the small ones gain.
     int ncta = 1;
-    while (ncta < kMaxCluster && ceil_div(G.max_nk, ncta) > kCacheSteps) ncta *= 2;
+    while (ncta < kMaxCluster &&
+           (ceil_div(G.max_nk, ncta) > kCacheSteps ||
+            (ceil_div(G.max_nk, ncta) > 2 && G.nitems * ncta * 2 <= 8 * ctx->num_sms)))
+      ncta *= 2;
     const int steps = (int)std::min<int64_t>(kCacheSteps, ceil_div(G.max_nk, ncta));
     const int smem = steps * BK * kPadRows * (int)sizeof(double);
     set_smem_limit_once(ctx, pack_set, pack_f64_kernel<MAP>,
