@@ -136,7 +136,7 @@ __global__ void __launch_bounds__(kSmallRows * kSmallCols) contract_small_kernel
 // (12 of its 34 allowed entries are not zero), a first term of 1.0 x is taken as x, and
 // several rows are in flight per thread. A row with a non-finite element does every FMA, as 0 x Inf
 // must give NaN. Measured, the MPO steps of a two-site H_eff with the copies that they replace:
-// chi = 2048 2 x 41 us (before 434), chi = 517 2 x 11 us (93).
+// chi = 2048 2 x 35 us (before 434), chi = 517 2 x 8 us (93).
 struct ThinShared {
   ThinOffset o[2 * kThinMax];    // K of the long operand, T of the output
   uint32_t mask[kThinMax];       // nonzero entries of a thin index
@@ -303,8 +303,8 @@ void plan_direct(const std::vector<MapProblem>& map, const std::vector<GemmTask>
     else tiled = true;
   }
   const bool small = fma <= kSmallFma && axes <= kSmallAxes && kmax <= kSmallK;
-  // rows per thin unit: about eight units per SM, so that staging a unit's tables is shared by
-  // many rows and the last wave is short
+  // rows per thin unit: about eight units per SM, so that staging a unit's tables is shared by many rows
+  // and the last wave is short (four or two: the chi = 1024 environment 125 -> 136, 155 us)
   const int64_t unit = std::min<int64_t>(
       2048, std::max<int64_t>(256, (thin_rows / (8 * num_sms) + 255) / 256 * 256));
   for (size_t p = 0; p < map.size(); ++p) {
@@ -473,8 +473,10 @@ bool launch_direct(Context* ctx, DirectPlan& p, const double* A, const double* B
       ctx->kernel_launches++;
     }
     if (p.nunits) {
-      // rows in flight per thread by the longest K, within 64 (K <= 8) or 128 registers
-      auto kern = p.thin_k <= 4   ? contract_thin_kernel<4, 4>
+      // Rows in flight per thread by the longest K. Two for K <= 4: with four (114 registers, two CTAs
+      // per SM) a two-site H_eff takes 98 us instead of 90 at chi = 517 and 536 instead of 523 at
+      // 2048, with one 540 there.
+      auto kern = p.thin_k <= 4   ? contract_thin_kernel<4, 2>
                   : p.thin_k <= 8 ? contract_thin_kernel<8, 2>
                   : p.thin_k <= 16 ? contract_thin_kernel<16, 1>
                                    : contract_thin_kernel<32, 1>;
