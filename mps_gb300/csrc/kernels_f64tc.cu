@@ -38,10 +38,11 @@
 // Measured: one 4096 x 4000 x 4096 product 2.72 ms (49 TFLOP/s of FP64 work, 74% of the bf16 rate in
 // digit products; the FP64 pipe takes 125 ms). Before the MMAs were issued from code that the
 // whole warp runs in step (elect_one) 3.72 ms: 80 cycles per MMA went into moving its operands to
-// uniform registers. The two GEMMs of a two-site H_eff, packing + this kernel: chi = 2048 141 + 323 us
-// (FP64 pipe 9205; tensor cycles 42 and 53%, the epilogue's integer sums and stores of a tile, 13000
-// cycles, hold the next one's MMAs up). Relative error of N(0,1) products against extended
-// precision: 2e-16 (K = 33) to 1.4e-15 (K = 2050) on the FP64 pipe, 5e-17 here.
+// uniform registers. A two-site H_eff (packing, this kernel, two thin
+// steps, packing, this kernel) takes 521 us at chi = 2048 (9680 on the FP64 pipe) and 89 us at chi = 517
+// (1005); at chi = 2048 this kernel is 2 x 160 us of it, tensor cycles 42 and 53%: the epilogue's integer
+// sums and stores of a tile, 13000 cycles, hold the next one's MMAs up. Relative error of N(0,1)
+// products against extended precision: 2e-16 (K = 33) to 1.4e-15 (K = 2050) on the FP64 pipe, 5e-17 here.
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 

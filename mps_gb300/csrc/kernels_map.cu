@@ -136,7 +136,8 @@ __global__ void __launch_bounds__(kSmallRows * kSmallCols) contract_small_kernel
 // (12 of its 34 allowed entries are not zero), a first term of 1.0 x is taken as x, and
 // several rows are in flight per thread. A row with a non-finite element does every FMA, as 0 x Inf
 // must give NaN. Measured, the MPO steps of a two-site H_eff with the copies that they replace:
-// chi = 2048 2 x 35 us (before 434), chi = 517 2 x 8 us (93).
+// chi = 2048 2 x 41 us (before 434), chi = 517 2 x 11 us (93), each with four rows in flight per thread
+// (launch_direct has the whole application with two, the faster choice).
 struct ThinShared {
   ThinOffset o[2 * kThinMax];    // K of the long operand, T of the output
   uint32_t mask[kThinMax];       // nonzero entries of a thin index

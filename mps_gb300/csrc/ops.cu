@@ -435,7 +435,8 @@ static const std::vector<int> kH4A = {1, 2, 3, -1, -2}, kH4B = {-2, -1, 4};
 
 // The arithmetic of a two-site H_eff. Five slices pay from about 4 GFLOP on, where the MMAs that they save
 // outweigh their extra passes (fused copies, exponents, W folded into the environments): FP64 / 5
-// slices in us, chi = 48 17 / 101, 517 106 / 172, 1024 194 / 254, 1448 330 / 334, 2048 549 / 466.
+// slices in us, chi = 48 17 / 101, 517 106 / 172, 1024 194 / 254, 1448 330 / 334, 2048 549 / 466 (since
+// then both faster by 5%, 521 / 442).
 // Smaller operators asked for with five slices get FP64 results. (Fewer slices are kept at every
 // size: a batch runs slices, and its operators agree with single ones to rounding there.)
 constexpr double kHeffFp64Flops = 4e9;
