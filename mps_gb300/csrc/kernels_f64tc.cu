@@ -744,7 +744,9 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f64tc_kernel(
 }
 
 constexpr size_t kGroupBytes = size_t(2) << 30;  // packed operands per launch pair
-constexpr int kMinPart = 3, kMaxParts = 16;      // K steps of a piece of a tile, pieces
+// Pieces of a tile. They may be as short as one K step: with three as the least, the chi = 363 right
+// environment takes 68.3 us instead of 65.8, a chi = 256 eigensolve 2.04 ms instead of 2.00.
+constexpr int kMaxParts = 16;
 // (with 1.5 for kCutSteps chi = 2048 takes 562 us instead of 549, chi = 517 the same)
 constexpr double kCutSteps = 2.5, kTileSteps = 1.0;
 
@@ -914,7 +916,7 @@ void plan_group(const std::vector<Task>& g, int num_sms, Group& G, GroupTables& 
   for (const Tile& x : t.tiles) max_nk = std::max<int64_t>(max_nk, x.ks1);
   double span = cut_at((int)max_nk, best, G.nslots), even = 0.0;
   for (const Tile& x : best) even += (x.ks1 - x.ks0 + kTileSteps) / num_sms;
-  for (int d = 2; d <= kMaxParts && ceil_div(max_nk, d) >= kMinPart && span > 1.1 * even; ++d) {
+  for (int d = 2; d <= kMaxParts && d <= max_nk && span > 1.1 * even; ++d) {
     const double s = cut_at((int)ceil_div(max_nk, d), cut, slots);
     if (s < 0.95 * span) {
       span = s;
