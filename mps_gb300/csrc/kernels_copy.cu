@@ -33,6 +33,7 @@
 #include <cstring>
 
 #include "copy_decode.hpp"
+#include "dep_load.cuh"
 #include "runtime.hpp"
 
 namespace mpsg {
@@ -377,7 +378,7 @@ __device__ __forceinline__ void bulk_issue(const BulkRow* rows, int64_t u, const
 // stops after draining the copies it has in flight (bounded as well; kBulkErrDrain if that
 // expires too).
 __global__ void __launch_bounds__(32 * kBulkWarps, 2) copy_rows_bulk_kernel(
-    const BulkRow* __restrict__ rows, int64_t nrows, const double* __restrict__ src,
+    const BulkRow* __restrict__ rows, int64_t nrows, const double* src,
     double* __restrict__ dst, int* __restrict__ err) {
   extern __shared__ __align__(128) unsigned char bulk_smem[];
   cudaTriggerProgrammaticLaunchCompletion();
@@ -396,6 +397,7 @@ __global__ void __launch_bounds__(32 * kBulkWarps, 2) copy_rows_bulk_kernel(
       asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&bars[s])));
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("fence.proxy.async.global;" ::: "memory");  // the source is the kernel before's output
     for (int64_t j = 0; j < mine && j < kBulkStages; ++j)
       bulk_issue(rows, first + j * W, src, slots + j * kSlotBytes, &bars[j]);
   }
@@ -428,16 +430,16 @@ __global__ void __launch_bounds__(32 * kBulkWarps, 2) copy_rows_bulk_kernel(
 #pragma unroll 4
       for (int i = lane; i < r.len; i += 32) {
         const uint64_t g = a0 + 8 * (uint64_t)i;
-        gdst[i] = (g >= i0 && g < i1) ? slot[(g - i0) >> 3] : __ldg(gsrc + i);
+        gdst[i] = (g >= i0 && g < i1) ? slot[(g - i0) >> 3] : load_dep(gsrc + i);
       }
     } else if (r.sstr == 1) {
       for (int i = lane; i < r.len; i += 32) {
         const uint64_t g = a0 + 8 * (uint64_t)i;
-        gdst[(int64_t)i * r.dstr] = (g >= i0 && g < i1) ? slot[(g - i0) >> 3] : __ldg(gsrc + i);
+        gdst[(int64_t)i * r.dstr] = (g >= i0 && g < i1) ? slot[(g - i0) >> 3] : load_dep(gsrc + i);
       }
     } else {  // a strided source row: plain loads
       for (int i = lane; i < r.len; i += 32)
-        gdst[(int64_t)i * r.dstr] = __ldg(gsrc + (int64_t)i * r.sstr);
+        gdst[(int64_t)i * r.dstr] = load_dep(gsrc + (int64_t)i * r.sstr);
     }
     __syncwarp();  // every lane has read the slot before it is refilled
     if (lane == 0 && j + kBulkStages < mine) {

@@ -49,6 +49,7 @@
 #include <algorithm>
 #include <type_traits>
 
+#include "dep_load.cuh"
 #include "f64tc.hpp"
 #include "tc5.cuh"
 
@@ -233,7 +234,7 @@ struct FusedCursor {
                                        double (&x)[kRun]) {
     const double* p = X + at0 + col * step;
 #pragma unroll
-    for (int j = 0; j < kRun; ++j) x[j] = col + j < end ? __ldg(p + j * step) : 0.0;
+    for (int j = 0; j < kRun; ++j) x[j] = col + j < end ? load_dep(p + j * step) : 0.0;
   }
 };
 
@@ -276,14 +277,14 @@ struct MapCursor {
       const double* p = X + at(e);
       const int64_t step = c0;
 #pragma unroll
-      for (int j = 0; j < kRun; ++j) x[j] = __ldg(p + j * step);
+      for (int j = 0; j < kRun; ++j) x[j] = load_dep(p + j * step);
       return;
     }
     int64_t a[kRun];
 #pragma unroll
     for (int j = 0; j < kRun; ++j) a[j] = col + j < end ? at(cols, col + j) : 0;
 #pragma unroll
-    for (int j = 0; j < kRun; ++j) x[j] = col + j < end ? __ldg(X + a[j]) : 0.0;
+    for (int j = 0; j < kRun; ++j) x[j] = col + j < end ? load_dep(X + a[j]) : 0.0;
   }
 };
 
@@ -303,10 +304,10 @@ template <Access MAP>
 __global__ void __launch_bounds__(256) pack_f64_kernel(
     const Problem* __restrict__ probs, const int2* __restrict__ items, int ncta, int cache_steps,
     const AxisEntry* __restrict__ axes, const MapBlock* __restrict__ blocks,
-    const double* __restrict__ A, const double* __restrict__ B, int32_t* __restrict__ RA,
+    const double* A, const double* B, int32_t* __restrict__ RA,
     int32_t* __restrict__ RB, __nv_bfloat16* __restrict__ packA, __nv_bfloat16* __restrict__ packB,
-    int64_t rowsA, int64_t rowsB, int* __restrict__ arrivals, ulonglong2* __restrict__ slots, int nslots, int64_t partA,
-    int64_t partB) {
+    int64_t rowsA, int64_t rowsB, int* __restrict__ arrivals, ulonglong2* __restrict__ slots,
+    int nslots, int64_t partA, int64_t partB) {
   extern __shared__ double xs[];  // [k][row], rows padded to kPadRows
   __shared__ uint32_t red[8][33], rlow[8][33];  // largest high words, all low words or-ed
   __shared__ uint2 rmax[kRowBlock];
@@ -369,7 +370,7 @@ __global__ void __launch_bounds__(256) pack_f64_kernel(
         Cursor<MAP> c(tab, row_ax + r0 + rr, x0, r0 + rr, rs, kstep, part);
 #pragma unroll 4
         for (int64_t k = kb + lane; k < ke; k += 32) {
-          const double x = __ldg(X + c.at(k_ax, k));
+          const double x = load_dep(X + c.at(k_ax, k));
           m = max(m, (uint32_t)__double2hiint(x) & 0x7fffffffu);
           lo |= (uint32_t)__double2loint(x);
           if (keep) xs[(int)(k - kb) * kPadRows + rr] = x;
@@ -508,9 +509,9 @@ template <Access MAP>
 __global__ void __launch_bounds__(kThreads, 1) gemm_f64tc_kernel(
     const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
     const Problem* __restrict__ probs, const Tile* __restrict__ tiles, int64_t ntiles,
-    const int32_t* __restrict__ RA, const int32_t* __restrict__ RB,
+    const int32_t* RA, const int32_t* RB,
     const AxisEntry* __restrict__ axes, const MapBlock* __restrict__ blocks,
-    const double* __restrict__ A, const double* __restrict__ B, double* __restrict__ C,
+    const double* A, const double* B, double* __restrict__ C,
     unsigned long long* __restrict__ slots, int* __restrict__ arrivals, int* __restrict__ err,
     const __grid_constant__ PartOffsets parts) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -552,6 +553,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f64tc_kernel(
   if (warp == 0) {
     // ---------------- TMA producer ----------------
     if (lane == 0) {
+      fence_proxy_async_global();
       int stage = 0;
       uint32_t phase = 0;
       for (int64_t i = 0; !*abort_flag; ++i) {

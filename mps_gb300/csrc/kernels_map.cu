@@ -5,6 +5,7 @@
 #include <algorithm>
 
 #include "copy_decode.hpp"
+#include "dep_load.cuh"
 #include "direct.hpp"
 
 namespace mpsg {
@@ -52,7 +53,7 @@ __device__ __forceinline__ int64_t mapped_at(const MapBlock* __restrict__ tab, c
 __global__ void __launch_bounds__(kSmallRows * kSmallCols) contract_small_kernel(
     const SmallProblem* __restrict__ probs, int nprob, int ntiles,
     const AxisEntry* __restrict__ axes, const MapBlock* __restrict__ blocks,
-    const double* __restrict__ A, const double* __restrict__ B, double* __restrict__ C,
+    const double* A, const double* B, double* __restrict__ C,
     const PartOffsets parts) {
   __shared__ double as[kChunk * kSmallRows], bs[kChunk * kSmallCols];
   const int4* ax = reinterpret_cast<const int4*>(axes);
@@ -95,10 +96,10 @@ __global__ void __launch_bounds__(kSmallRows * kSmallCols) contract_small_kernel
       double va[kA], vb[kB];
 #pragma unroll
       for (int u = 0; u < kB; ++u)
-        if ((t >> 2) + kSmallRows * u < kn) vb[u] = __ldg(B + ob[u]);
+        if ((t >> 2) + kSmallRows * u < kn) vb[u] = load_dep(B + ob[u]);
 #pragma unroll
       for (int u = 0; u < kA; ++u)
-        if (w + kSmallCols * u < kn) va[u] = __ldg(A + oa[u]);
+        if (w + kSmallCols * u < kn) va[u] = load_dep(A + oa[u]);
       if (c0 > 0 || tile != blockIdx.x) __syncthreads();  // the last chunk has been read
 #pragma unroll
       for (int u = 0; u < kA; ++u)
@@ -107,7 +108,7 @@ __global__ void __launch_bounds__(kSmallRows * kSmallCols) contract_small_kernel
 #pragma unroll
         for (int u = 0; u < kA; ++u) {
           const int k = kPart + w + kSmallCols * u;
-          if (k < kn) va[u] = __ldg(A + mapped_at(ta, me, __ldg(ke + k), parts.a));
+          if (k < kn) va[u] = load_dep(A + mapped_at(ta, me, __ldg(ke + k), parts.a));
         }
 #pragma unroll
         for (int u = 0; u < kA; ++u) {
@@ -174,7 +175,7 @@ __device__ __forceinline__ void thin_terms(double (&acc)[ROWS], const double (&a
 // inside the unit).
 template <int KMAX, int ROWS>
 __device__ __forceinline__ void thin_rows(const ThinShared& s, const ThinUnit& u, int row,
-                                          const double* __restrict__ X, double* __restrict__ C) {
+                                          const double* X, double* __restrict__ C) {
   const int K = u.K;
   int i0[ROWS], i1[ROWS], i2[ROWS];
   bool in[ROWS];
@@ -194,7 +195,7 @@ __device__ __forceinline__ void thin_rows(const ThinShared& s, const ThinUnit& u
       const ThinOffset o = s.o[k];
 #pragma unroll
       for (int y = 0; y < ROWS; ++y)
-        a[y][k] = __ldg(X + o.off + (i0[y] * o.rs0 + i1[y] * o.rs1 + i2[y] * o.rs2));
+        a[y][k] = load_dep(X + o.off + (i0[y] * o.rs0 + i1[y] * o.rs1 + i2[y] * o.rs2));
     } else {
 #pragma unroll
       for (int y = 0; y < ROWS; ++y) a[y][k] = 0.0;
@@ -240,7 +241,7 @@ __device__ __forceinline__ void thin_rows(const ThinShared& s, const ThinUnit& u
 template <int KMAX, int ROWS>
 __global__ void __launch_bounds__(256) contract_thin_kernel(
     const ThinUnit* __restrict__ units, int nunits, const ThinOffset* __restrict__ offs,
-    const int64_t* __restrict__ vals, const double* __restrict__ A, const double* __restrict__ B,
+    const int64_t* __restrict__ vals, const double* A, const double* B,
     double* __restrict__ C, const PartOffsets parts) {
   __shared__ ThinShared s;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -258,7 +259,8 @@ __global__ void __launch_bounds__(256) contract_thin_kernel(
     }
     if (it == blockIdx.x) cudaGridDependencySynchronize();
     for (int x = threadIdx.x; x < u.T * u.K; x += blockDim.x)
-      s.b[x] = __ldg(S + part_base(__ldg(vals + u.vals + x), u.longB ? parts.a : parts.b, 0, 0));
+      s.b[x] =
+          load_dep(S + part_base(__ldg(vals + u.vals + x), u.longB ? parts.a : parts.b, 0, 0));
     __syncthreads();
     if (threadIdx.x < u.T) {
       const double* b = s.b + threadIdx.x * u.K;
@@ -440,8 +442,7 @@ DirectPlan::~DirectPlan() {
 // in one pass and launch.
 __global__ void __launch_bounds__(256) complex_parts_kernel(int64_t n, double* __restrict__ rr,
                                                             double* __restrict__ ri,
-                                                            const double* __restrict__ ir,
-                                                            const double* __restrict__ ii,
+                                                            const double* ir, const double* ii,
                                                             double c_ri, double c_ir, double c_ii) {
   cudaTriggerProgrammaticLaunchCompletion();
   cudaGridDependencySynchronize();

@@ -38,6 +38,7 @@
 #include <cstring>
 #include <type_traits>
 
+#include "dep_load.cuh"
 #include "split.hpp"
 #include "tc5.cuh"
 
@@ -188,7 +189,7 @@ constexpr int kExpRowsA = 32, kExpRowsB = 32;
 
 __global__ void __launch_bounds__(256) pack_exponents_kernel(
     const Problem* __restrict__ probs, const int64_t* __restrict__ item_prefix, int nprob,
-    int64_t nitems, int is_b, int chunk, int write_e, const double* __restrict__ X,
+    int64_t nitems, int is_b, int chunk, int write_e, const double* X,
     int16_t* __restrict__ E,
     int32_t* __restrict__ R) {
   __shared__ unsigned long long red[8][33];
@@ -266,7 +267,7 @@ template <int S>
 __global__ void __launch_bounds__(256) pack_slices_kernel(
     const Problem* __restrict__ probs, const int64_t* __restrict__ tile_prefix, int nprob,
     int64_t ntiles, int is_b, int chunk, int use_r, int rows_per_tile, int64_t rows_total,
-    const double* __restrict__ X, const int16_t* __restrict__ E, const int32_t* __restrict__ R,
+    const double* X, const int16_t* E, const int32_t* R,
     __nv_bfloat16* __restrict__ out) {
   constexpr int kBeta = kSliceBits;
   cudaTriggerProgrammaticLaunchCompletion();
@@ -296,7 +297,7 @@ __global__ void __launch_bounds__(256) pack_slices_kernel(
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
           const int64_t k = k0 + g8 * 8 + j;
-          xv[j] = (r < rows && k < P.K) ? __ldg(X + off + r * rs + k * ks) : 0.0;
+          xv[j] = (r < rows && k < P.K) ? load_dep(X + off + r * rs + k * ks) : 0.0;
         }
         int e = 0, Rr = 0;
         if (r < rows) {
@@ -415,7 +416,7 @@ template <int S, int BN>
 __global__ void __launch_bounds__(kExactThreads, 1) split_gemm_kernel(
     const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
     const Problem* __restrict__ probs, const int4* __restrict__ tiles, int64_t ntiles,
-    const int32_t* __restrict__ RA, const int32_t* __restrict__ CB, double* __restrict__ C,
+    const int32_t* RA, const int32_t* CB, double* __restrict__ C,
     int* __restrict__ err) {
   using CF = Cfg<S, BN>;
   static_assert(CF::kThreads == kExactThreads, "launch bound and epilogue warp count disagree");
@@ -455,6 +456,7 @@ __global__ void __launch_bounds__(kExactThreads, 1) split_gemm_kernel(
   if (warp == 0) {
     // ---------------- TMA producer ----------------
     if (lane == 0) {
+      fence_proxy_async_global();
       int stage = 0;
       uint32_t phase = 0;
       for (int64_t i = 0; !*abort_flag; ++i) {
@@ -666,7 +668,7 @@ template <int S>
 __global__ void __launch_bounds__(192, 1) split_gemm_fast_kernel(
     const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
     const Problem* __restrict__ probs, const int4* __restrict__ tiles, int64_t ntiles,
-    const int32_t* __restrict__ RA, const int32_t* __restrict__ CB, double* __restrict__ C,
+    const int32_t* RA, const int32_t* CB, double* __restrict__ C,
     int* __restrict__ err) {
   using CF = FastCfg<S>;
   extern __shared__ __align__(1024) uint8_t smem_raw[];
@@ -705,6 +707,7 @@ __global__ void __launch_bounds__(192, 1) split_gemm_fast_kernel(
   if (warp == 0) {
     // ---------------- TMA producer ----------------
     if (lane == 0) {
+      fence_proxy_async_global();
       int stage = 0;
       uint32_t phase = 0;
       for (int64_t i = 0; !*abort_flag; ++i) {

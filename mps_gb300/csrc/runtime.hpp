@@ -30,6 +30,11 @@ namespace mpsg {
 // tables uploaded before that kernel and call cudaGridDependencySynchronize() before they touch anything
 // else, every block of them (so that one kernel's end implies the end of all before it). Kernels
 // launched so also let their successor start (cudaTriggerProgrammaticLaunchCompletion).
+// Such a kernel is alive while its predecessor writes its operands, and the read-only data path is only
+// for memory that nobody writes while the kernel lives: what a kernel before may have written is read with
+// ordinary loads (load_dep) through pointers that are not const __restrict__ (__ldg, or the two qualifiers,
+// allow that path, and let the compiler move a load above the wait). Tables written by uploads may use
+// it: an upload between two kernels keeps the second from starting early.
 // Measured with the launches of a contraction chained so, two-site H_eff: chi = 48 42 -> 30 us (4 launches),
 // chi = 517 122 -> 114 us (6), a chi = 64 DMRG sweep of 32 sites 112 -> 99 ms;
 // with five slices, chi = 2048, 466 -> 441 us (11; a chained kernel in place of the memsets: 451).
