@@ -53,6 +53,12 @@ int mpsg_ctx_synchronize(mpsg_ctx* ctx);
 /* Counters: kernels launched by this library and algorithmic block-GEMM flops issued. */
 int mpsg_ctx_counters(mpsg_ctx* ctx, int64_t* kernel_launches, double* gemm_flops);
 int mpsg_ctx_clear_caches(mpsg_ctx* ctx);
+/* Every wait inside a kernel is bounded. A kernel of the FP64 products or of the Krylov solver whose wait
+ * expires ends without its results, and the next call on the context that synchronises to return host
+ * values (downloads, dots, scalars, singular values, eigsolve, mpsg_ctx_synchronize) fails with
+ * MPSG_ERR_CUDA; the record is then cleared. mpsg_ctx_record_wait makes that record from a kernel on the
+ * context's stream (which: 0 = FP64 product, 1 = Krylov solver), to test the callers of a program. */
+int mpsg_ctx_record_wait(mpsg_ctx* ctx, int32_t which, int32_t code);
 /* Debug library only (libmpsgb300_checked.so, built with MPSG_DEVICE_CHECKS): the copy kernel
  * recomputes every block offset it decodes by plain division, checks every address against its
  * task's span, and records a violation instead of making the access (no counterpart in the

@@ -71,6 +71,7 @@ SIGNATURES = {
     "mpsg_tensor_download": [P, PF64, I64],
     "mpsg_tensor_device_ptr": [P, PP],
     "mpsg_device_checks": [P, I32, PI64, PI64],
+    "mpsg_ctx_record_wait": [P, I32, I32],
     "mpsg_host_alloc": [I64, PP],
     "mpsg_host_free": [P],
     "mpsg_tensor_download_async": [P, P, P, I64, PP],

@@ -708,6 +708,7 @@ std::vector<EigResult> eigsolve_heff2_batch(HeffBatch& B, const std::vector<cons
     launched(2);
     MPSG_CUDA(cudaMemcpyAsync(h_out, out, sizeof(double) * nch, cudaMemcpyDeviceToHost, st));
     MPSG_CUDA(cudaStreamSynchronize(st));
+    check_waits(ctx);
   };
   auto orthogonalize = [&](const StepArgs& a) {
     for (int pass = 0; pass < 2; ++pass) {

@@ -73,6 +73,7 @@ int mpsg_ctx_synchronize(mpsg_ctx* ctx) {
   return guarded([&] {
     need(ctx, "ctx");
     MPSG_CUDA(cudaStreamSynchronize(ctx->c.stream));
+    mpsg::check_waits(&ctx->c);
   });
 }
 
@@ -226,6 +227,16 @@ int mpsg_tensor_download(const mpsg_tensor* t, double* host, int64_t n) {
     MPSG_CUDA(cudaMemcpyAsync(host, t->t.data(), sizeof(double) * n, cudaMemcpyDeviceToHost,
                               t->t.ctx->stream));
     MPSG_CUDA(cudaStreamSynchronize(t->t.ctx->stream));
+    mpsg::check_waits(t->t.ctx);
+  });
+}
+
+int mpsg_ctx_record_wait(mpsg_ctx* ctx, int32_t which, int32_t code) {
+  return guarded([&] {
+    need(ctx, "ctx");
+    if (which != mpsg::kWaitGemm && which != mpsg::kWaitKrylov)
+      throw mpsg::Error(mpsg::kErrArgument, "record_wait: which must be 0 or 1");
+    mpsg::launch_record_wait(&ctx->c, which, code);
   });
 }
 
@@ -305,6 +316,7 @@ int mpsg_copy_query(mpsg_copy* copy, int32_t* done) {
       return;
     }
     MPSG_CUDA(e);
+    mpsg::check_waits(copy->c->owner.get());
     *done = 1;
   });
 }
@@ -313,6 +325,7 @@ int mpsg_copy_synchronize(mpsg_copy* copy) {
   return guarded([&] {
     need(copy, "copy");
     MPSG_CUDA(cudaEventSynchronize(copy->c->done));
+    mpsg::check_waits(copy->c->owner.get());
   });
 }
 

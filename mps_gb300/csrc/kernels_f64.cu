@@ -432,6 +432,14 @@ void dots_host(Context* ctx, const std::vector<VecPair>& pairs, double* out) {
   MPSG_CUDA(cudaFreeAsync(d_pairs, st));
   MPSG_CUDA(cudaFreeAsync(d_part, st));
   MPSG_CUDA(cudaStreamSynchronize(st));
+  check_waits(ctx);
+}
+
+static __global__ void record_wait_kernel(int* err, int code) { record_wait(err, code); }
+
+void launch_record_wait(Context* ctx, int which, int code) {
+  record_wait_kernel<<<1, 1, 0, ctx->stream>>>(ctx->wait_err + which, code);
+  MPSG_CUDA(cudaGetLastError());
 }
 
 void launch_lincomb(Context* ctx, int64_t n, const std::vector<const double*>& xs,

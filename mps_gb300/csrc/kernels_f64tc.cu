@@ -1032,7 +1032,7 @@ static void launch_group(Context* ctx, Group& G, unsigned char* mem, const doubl
   const int grid = (int)std::min<int64_t>(G.ntiles, ctx->num_sms);
   launch_chained(gemm_f64tc_kernel<MAP>, dim3((unsigned)grid), dim3(kThreads), (size_t)kSmemBytes, st,
                  1, tmA, tmB, G.d_probs, G.d_tiles, G.ntiles, RA, RB, G.d_axes, G.d_blocks, A, B, C,
-                 slots, arrivals, ctx->d_tc_err, parts);
+                 slots, arrivals, ctx->wait_err + kWaitGemm, parts);
   ctx->kernel_launches++;
 }
 
@@ -1062,14 +1062,8 @@ bool launch(Context* ctx, Plan& p, const double* A, const double* B, double* C,
     MPSG_CUDA(cudaFreeAsync(mem, st));
   }
   if (ctx->debug_sync) {
-    int code = 0;
-    MPSG_CUDA(cudaMemcpyAsync(&code, ctx->d_tc_err, sizeof(int), cudaMemcpyDeviceToHost, st));
     MPSG_CUDA(cudaStreamSynchronize(st));
-    if (code) {
-      MPSG_CUDA(cudaMemsetAsync(ctx->d_tc_err, 0, sizeof(int), st));
-      throw Error(kErrCuda, "FP64 tensor-core GEMM: a bounded wait expired (role code " +
-                                std::to_string(code) + ")");
-    }
+    check_waits(ctx);
   }
   return true;
 }

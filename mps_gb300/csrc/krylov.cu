@@ -9,7 +9,6 @@
 
 #include <algorithm>
 #include <cmath>
-#include <cstring>
 
 #include "linalg.hpp"
 
@@ -97,7 +96,7 @@ __device__ __forceinline__ void grid_barrier(const GridBarrier& b, int i) {
     const long long t0 = clock64();
     while ((int)(*(volatile unsigned*)b.count - target) < 0)
       if (clock64() - t0 > kBarrierCycles) {
-        atomicCAS(b.err, 0, 1);
+        record_wait(b.err, 1);
         break;
       }
     __threadfence();
@@ -312,7 +311,6 @@ struct LanczosWork {
   std::shared_ptr<Buffer> buf;
   double *part, *out;     // partial sums; per step of a cycle (alpha, beta), then the start norm
   unsigned* count;
-  int* err;
   LanczosWork(Context* c, int kd_, int64_t n_) : ctx(c), kd(kd_), n(n_) {
     // one block per SM at most: co-resident, and few arrivals per barrier; short vectors are bound
     // by the FP64 pipes of the SMs that take part (22 FMAs per element at K = 5), so they spread
@@ -321,15 +319,15 @@ struct LanczosWork {
     cluster = n <= (int64_t)kClusterBlocks * kClusterRows * kVecThreads;
     if (cluster) grid = std::min(grid, kClusterBlocks);
     const int64_t np = 3 * (int64_t)kd * grid;
-    buf = alloc_buffer(ctx, np + 2 * kd + 4);
+    buf = alloc_buffer(ctx, np + 2 * kd + 3);
     part = buf->ptr;
     out = part + np;
     count = (unsigned*)(out + 2 * kd + 2);
-    err = (int*)(out + 2 * kd + 3);
-    MPSG_CUDA(cudaMemsetAsync(count, 0, 2 * sizeof(double), ctx->stream));
+    MPSG_CUDA(cudaMemsetAsync(count, 0, sizeof(double), ctx->stream));
   }
   GridBarrier barrier(int n_barriers) {
-    GridBarrier b{cluster ? nullptr : count, (barriers + 1) * (unsigned)grid, err};
+    GridBarrier b{cluster ? nullptr : count, (barriers + 1) * (unsigned)grid,
+                  ctx->wait_err + kWaitKrylov};
     barriers += (unsigned)n_barriers;
     return b;
   }
@@ -391,12 +389,10 @@ struct LanczosWork {
   }
   // (alpha, beta) of the cycle's steps and the start norm, in the context's pinned scratch
   const double* read() {
-    MPSG_CUDA(cudaMemcpyAsync(ctx->h_pinned, out, sizeof(double) * (2 * kd + 4),
+    MPSG_CUDA(cudaMemcpyAsync(ctx->h_pinned, out, sizeof(double) * (2 * kd + 1),
                               cudaMemcpyDeviceToHost, ctx->stream));
     MPSG_CUDA(cudaStreamSynchronize(ctx->stream));
-    int e = 0;
-    std::memcpy(&e, ctx->h_pinned + 2 * kd + 3, sizeof(int));
-    if (e) throw Error(kErrCuda, "eigsolve: a bounded wait between blocks expired");
+    check_waits(ctx);
     return ctx->h_pinned;
   }
 };

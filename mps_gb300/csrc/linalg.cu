@@ -564,6 +564,7 @@ SVDResult svd_blocks(Context* ctx, const DeviceTensor& A, bool truncate, int64_t
     MPSG_CUDA(cudaMemcpyAsync(host.data(), values->ptr, sizeof(double) * host.size(),
                               cudaMemcpyDeviceToHost, ctx->stream));
     MPSG_CUDA(cudaStreamSynchronize(ctx->stream));
+    check_waits(ctx);
     std::memcpy(info.data(), host.data() + nS, sizeof(int) * nb);
     for (size_t b = 0; b < nb; ++b)
       S[b].assign(host.begin() + blocks[b].offS, host.begin() + blocks[b].offS + blocks[b].k);
@@ -732,6 +733,7 @@ CSVDResult svd_blocks_complex(Context* ctx, const DeviceTensor& Are, const Devic
   }
   MPSG_CUDA(cudaStreamSynchronize(ctx->stream));
   if (dinfo) cudaFreeAsync(dinfo, ctx->stream);
+  check_waits(ctx);
   for (size_t b = 0; b < nb; ++b)
     if (info[b] != 0) throw Error(kErrNoConvergence, "complex block SVD did not converge");
   int64_t total = 0;

@@ -37,10 +37,11 @@ void context_init(Context* ctx, int device) {
   uint64_t thr = UINT64_MAX;  // keep freed blocks cached in the pool
   MPSG_CUDA(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &thr));
   MPSG_CUDA(cudaMalloc(&ctx->d_partials, sizeof(double) * (ctx->num_sms * 4 + 64)));
-  MPSG_CUDA(cudaMalloc(&ctx->d_copy_err, 2 * sizeof(int)));
-  MPSG_CUDA(cudaMemset(ctx->d_copy_err, 0, 2 * sizeof(int)));
-  ctx->d_tc_err = ctx->d_copy_err + 1;
+  MPSG_CUDA(cudaMalloc(&ctx->d_copy_err, sizeof(int)));
+  MPSG_CUDA(cudaMemset(ctx->d_copy_err, 0, sizeof(int)));
   MPSG_CUDA(cudaMallocHost(&ctx->h_pinned, sizeof(double) * Context::kPinnedDoubles));
+  ctx->wait_err = (int*)(ctx->h_pinned + Context::kPinnedDoubles - 1);
+  ctx->wait_err[kWaitGemm] = ctx->wait_err[kWaitKrylov] = 0;
   const char* dbg = std::getenv("MPSG_DEBUG_SYNC");
   ctx->debug_sync = dbg && dbg[0] == '1';
 }
@@ -67,6 +68,16 @@ KernelTimer::~KernelTimer() {
   if (!a) return;
   cudaEventRecord(b, ctx->stream);
   ctx->events[kind].push_back({a, b, flops});
+}
+
+void check_waits(Context* ctx) {
+  volatile int* w = ctx->wait_err;
+  const int gemm = w[kWaitGemm], krylov = w[kWaitKrylov];
+  if (gemm == 0 && krylov == 0) return;
+  w[kWaitGemm] = w[kWaitKrylov] = 0;
+  throw Error(kErrCuda, gemm ? "FP64 tensor-core GEMM: a bounded wait expired (role code " +
+                                   std::to_string(gemm) + ")"
+                             : std::string("eigsolve: a bounded wait between blocks expired"));
 }
 
 void collect_kernel_times(Context* ctx) {
@@ -398,6 +409,7 @@ DeviceTensor contract(Context* ctx, const DeviceTensor& a, const std::vector<int
       MPSG_CUDA(cudaMemcpyAsync(ctx->h_pinned, ctx->d_partials + ctx->num_sms * 4,
                                 sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
       MPSG_CUDA(cudaStreamSynchronize(ctx->stream));
+      check_waits(ctx);
       s = ctx->h_pinned[0];
     }
     if (scalar) *scalar = s;
@@ -545,6 +557,7 @@ DeviceTensor applymps2site_host(Context* ctx, const DeviceTensor& v, const Devic
     MPSG_CUDA(cudaMemcpyAsync(host_out, out.data(), sizeof(double) * out.meta.total,
                               cudaMemcpyDeviceToHost, ctx->stream));
   MPSG_CUDA(cudaStreamSynchronize(ctx->stream));
+  check_waits(ctx);
   return out;
 }
 
@@ -835,6 +848,7 @@ double dot(Context* ctx, const DeviceTensor& a, const DeviceTensor& b) {
   MPSG_CUDA(cudaMemcpyAsync(ctx->h_pinned, d_out, sizeof(double), cudaMemcpyDeviceToHost,
                             ctx->stream));
   MPSG_CUDA(cudaStreamSynchronize(ctx->stream));
+  check_waits(ctx);
   return ctx->h_pinned[0];
 }
 

@@ -222,9 +222,12 @@ struct Context : std::enable_shared_from_this<Context> {
   cudaStream_t stream = nullptr;
   double* d_partials = nullptr;   // reduction partials (one per CTA of a reduction launch)
   int* d_copy_err = nullptr;      // set by the TMA-staged copy kernel when a bounded wait expires
-  int* d_tc_err = nullptr;        // ... and by the FP64 tensor-core GEMM
+  // Where kernels of the default paths record a bounded wait that expired (record_wait): words of the
+  // pinned scratch, so that the host has them after any synchronisation (check_waits).
+  int* wait_err = nullptr;        // [kWaitGemm], [kWaitKrylov]
   // small pinned host scratch: [0, 64) scalar results, [64, 64 + 3 * 128) the batched Lanczos
-  static constexpr int kPinnedDoubles = 64 + 3 * 128;
+  // and the wait_err words
+  static constexpr int kPinnedDoubles = 64 + 3 * 128 + 1;
   double* h_pinned = nullptr;
   PlanCache<DevContract> contract_cache;
   std::unordered_map<std::string, std::shared_ptr<DevReleg>> releg_cache;
@@ -261,6 +264,18 @@ struct Context : std::enable_shared_from_this<Context> {
   double timed_flops[kKinds] = {0, 0, 0, 0, 0, 0};
   ~Context();
 };
+
+// Raises (and clears) what kernels recorded in ctx->wait_err. Called after every synchronisation of the
+// context's stream that returns values to the host: a kernel whose wait expired ends without having
+// written its results, and nothing computed from them leaves the device as if they were good.
+enum { kWaitGemm = 0, kWaitKrylov = 1 };
+void check_waits(Context* ctx);
+void launch_record_wait(Context* ctx, int which, int code);  // as an expired wait does (tests)
+#ifdef __CUDACC__
+__device__ __forceinline__ void record_wait(int* err, int code) {
+  *(volatile int*)err = code;  // (pinned host memory: a store, not an atomic)
+}
+#endif
 
 enum KernelKind {
   kKindCopy = 0,

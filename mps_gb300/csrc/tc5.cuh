@@ -58,7 +58,7 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
     if (*abort_flag) return false;
     if (clock64() - t0 > kWaitCycles) {
       *abort_flag = 1;
-      atomicCAS(err, 0, code);
+      *(volatile int*)err = code;  // (may be host memory)
       return false;
     }
   }
