@@ -11,12 +11,13 @@
 namespace mpsg {
 namespace f64tc {
 
-constexpr int BM = 128, BN = 80, BK = 32;  // output tile and K step
-constexpr int kSlices = 7;                 // 9-bit digits of a 61-bit fixed-point operand
+constexpr int BM = 128, BN = 64, BK = 32;  // output tile and K step
+constexpr int kSlices = 9;                 // 9-bit digits of a 79-bit fixed-point operand
+constexpr int kFewSlices = 7;              // the leading ones, which most tiles need
 constexpr int64_t kMaxK = 65536;           // whole K summed in 64 bits (fits up to 2^22)
 
 // One sector GEMM as the kernels see it: R is the operand on the 128-row side, S the one on the
-// 80-row side. Either operand of the contraction may be R (swap: it is B, and the output is written
+// 64-row side. Either operand of the contraction may be R (swap: it is B, and the output is written
 // transposed), see plan_group. Elements are found by strides (fused matrices) or, in a
 // mapped group, by axis entries and block tables (the tensors themselves).
 struct Problem {
@@ -25,6 +26,7 @@ struct Problem {
   int64_t ob, brs, bks;       // element (n, k) of S
   int64_t oc, crs, ccs;       // output (m, n)
   int64_t tA, tB, rA, rB;     // first packed tile and first exponent entry of each operand
+  int32_t lA, lB;             // first count of large elements (one per 32 rows), R and S
   int32_t mt, nt, nk, swap;   // M tiles, N tiles, K steps
   int32_t axM, axN, axK;      // mapped: first axis entry of the rows of R, of S and of k
   int32_t blkA, blkB, blkC;   // ... first block of R [row combo][k combo], of S, of the output
@@ -34,16 +36,20 @@ struct Problem {
 
 // One output tile, or one of `parts` pieces of its K steps: the pieces add their sums to scratch slot
 // `slot` and the last one to arrive writes the tile.
-struct Tile {
+struct alignas(16) Tile {
   int32_t prob, mi, ni, ks0, ks1;  // K steps [ks0, ks1)
-  int32_t slot, part, parts;
+  int32_t slot, parts;
+  int32_t K;                       // of the problem
+  int32_t lA, lB, nA, nB;          // counts of large elements of its rows: first and number, R and S
+  int32_t rowA, rowB;              // first packed row of K step 0, R and S
 };
 
 // Problems that are packed and multiplied by one pair of launches (their packed operands share
 // one scratch allocation of at most about kGroupBytes, more only for a single larger problem).
 struct Group {
   int nprob = 0, nitems = 0, max_nk = 0;
-  int64_t ntiles = 0, nslots = 0, rowsA = 0, rowsB = 0, rA = 0, rB = 0;
+  int64_t ntiles = 0, ntiles_k = 0;  // ntiles_k: those with K steps, which come first
+  int64_t nslots = 0, rowsA = 0, rowsB = 0, rA = 0, rB = 0, lA = 0, lB = 0;
   double flops = 0;
   unsigned char* d_tables = nullptr;  // problems, output tiles, packing items
   Problem* d_probs = nullptr;

@@ -233,8 +233,8 @@ DeviceTensor symmatrix(Context* ctx, const DeviceTensor& a, const std::vector<in
 // block GEMM dispatch
 // ------------------------------------------------------------------------------------------
 // The arithmetic that a precision argument runs with: from 6 slices on the FP64 products of the
-// tensor cores (seven 9-bit slices, exact to the last bit of FP64), which are as many or fewer MMAs than
-// the 6- and 7-slice split products (1e-12 and 1e-14).
+// tensor cores (9-bit digits, 28 to 45 products, no element less accurate than FP64 FMAs make it), where the 6-
+// and 7-slice split products take 21 and 28 and passes of their own for 1e-12 and 1e-14.
 static int arithmetic(int precision) {
   if (precision == 0 || (precision >= 2 && precision < kFp64Slices)) return precision;
   if (precision >= kFp64Slices && precision <= split::kMaxSlices) return 0;
