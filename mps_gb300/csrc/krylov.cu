@@ -4,7 +4,7 @@
 //
 // Measured, ground-state solve at chi = 256 (19 products, krylovdim 5, 8 cycles): 4.6 ms with a dozen
 // launches and one host synchronisation per step and the projected matrix decomposed by one warp
-// (112 us a cycle), 2.6 ms with one launch per step (21 us) and one synchronisation per cycle.
+// (112 us a cycle), 2.6 ms with one launch per step (21 us) and the host kLag steps behind.
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -309,7 +309,8 @@ struct LanczosWork {
   bool cluster;
   unsigned barriers = 0;
   std::shared_ptr<Buffer> buf;
-  double *part, *out;     // partial sums; per step of a cycle (alpha, beta), then the start norm
+  double* part;           // partial sums
+  double* out;            // pinned: per step of a cycle (alpha, beta), then the norm of a combination
   unsigned* count;
   LanczosWork(Context* c, int kd_, int64_t n_) : ctx(c), kd(kd_), n(n_) {
     // one block per SM at most: co-resident, and few arrivals per barrier; short vectors are bound
@@ -319,10 +320,12 @@ struct LanczosWork {
     cluster = n <= (int64_t)kClusterBlocks * kClusterRows * kVecThreads;
     if (cluster) grid = std::min(grid, kClusterBlocks);
     const int64_t np = 3 * (int64_t)kd * grid;
-    buf = alloc_buffer(ctx, np + 2 * kd + 3);
+    buf = alloc_buffer(ctx, np + 1);
     part = buf->ptr;
-    out = part + np;
-    count = (unsigned*)(out + 2 * kd + 2);
+    out = ctx->h_pinned + Context::kPinnedKrylov;
+    count = (unsigned*)(part + np);
+    for (auto& e : ctx->krylov_ev)
+      if (!e) MPSG_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     MPSG_CUDA(cudaMemsetAsync(count, 0, sizeof(double), ctx->stream));
   }
   GridBarrier barrier(int n_barriers) {
@@ -387,23 +390,28 @@ struct LanczosWork {
     MPSG_CUDA(cudaGetLastError());
     ctx->kernel_launches++;
   }
-  // (alpha, beta) of the cycle's steps and the start norm, in the context's pinned scratch
-  const double* read() {
-    MPSG_CUDA(cudaMemcpyAsync(ctx->h_pinned, out, sizeof(double) * (2 * kd + 1),
-                              cudaMemcpyDeviceToHost, ctx->stream));
-    MPSG_CUDA(cudaStreamSynchronize(ctx->stream));
+  // The end of what has been queued so far, as number i, and the wait for it (at most kLag + 1 later ones may
+  // have been marked by then). Kernels write their results into pinned memory, where they are after the wait.
+  static constexpr int kLag = 2;
+  static_assert(kLag + 1 < sizeof(Context::krylov_ev) / sizeof(cudaEvent_t), "events in flight");
+  void mark(int i) { MPSG_CUDA(cudaEventRecord(ctx->krylov_ev[i & 3], ctx->stream)); }
+  void wait(int i) {
+    MPSG_CUDA(cudaEventSynchronize(ctx->krylov_ev[i & 3]));
     check_waits(ctx);
-    return ctx->h_pinned;
   }
+  double alpha(int i) const { return ((volatile double*)out)[2 * i]; }
+  double beta(int i) const { return ((volatile double*)out)[2 * i + 1]; }
+  double norm() const { return ((volatile double*)out)[2 * kd]; }
 };
 
 }  // namespace
 
-// The recurrence runs ahead on the device: matrix-vector products and Krylov steps are queued for a
-// whole cycle (krylovdim - kept vectors of them), and the host reads the cycle's coefficients
-// once, decomposes the projected matrix (a few us for its at most 32 x 32 elements) and decides. A
-// step whose remainder is below tol ends the solve at that step; what was queued after it is
-// dropped.
+// The recurrence runs ahead on the device: matrix-vector products and Krylov steps are queued while the host
+// looks at the coefficients of the step kLag before, so the device does not wait for it, and a start
+// vector that is refused or a step whose remainder is below tol (which ends the solve at that step) is
+// known at most kLag products later; what was queued after it is dropped. At the end of a cycle (krylovdim -
+// kept vectors of products) the host decomposes the projected matrix (a few us for its at most 32 x 32
+// elements) and decides.
 EigResult eigsolve_heff2(Context* ctx, const DeviceTensor& x0, const DeviceTensor& envL,
                          const DeviceTensor& envR, const DeviceTensor& W1, const DeviceTensor& W2,
                          int krylovdim, int maxiter, double tol, int precision) {
@@ -418,21 +426,32 @@ EigResult eigsolve_heff2(Context* ctx, const DeviceTensor& x0, const DeviceTenso
   for (int j = 0; j <= kd; ++j) V.push_back(new_tensor(ctx, x0.meta, false));
   const double one = 1.0;
   Wk.combine({x0.data()}, &one, V[0].data());
+  Wk.mark(3);  // (its event is not reused before step 3)
   std::vector<double> H(kd * kd, 0.0), D(kd), U(kd * kd);  // column-major, leading dimension kd
   auto at = [&](int i, int j) -> double& { return H[i + kd * j]; };
   int have = 1, numops = 0;  // basis vectors at the cycle's start (the newest not yet multiplied)
   for (int numiter = 1;; ++numiter) {
-    for (int K = have; K <= kd; ++K) {
+    bool more = true;
+    for (int K = have; K <= kd && more; ++K) {
+      const int i = K - have, before = i - LanczosWork::kLag;
       DeviceTensor w = heff_apply(*op, V[K - 1]);
-      Wk.step(K - have, V, K, w, V[K]);
+      Wk.step(i, V, K, w, V[K]);
+      Wk.mark(i);
+      if (before >= 0) {
+        Wk.wait(before);
+        more = Wk.beta(before) > tol || std::isnan(Wk.beta(before));
+      }
+      if (numiter == 1 && i == 0) {
+        MPSG_CUDA(cudaEventSynchronize(ctx->krylov_ev[3]));
+        if (!(Wk.norm() > 0)) throw Error(kErrArgument, "eigsolve: zero start vector");
+      }
+      if (K == kd || !more) Wk.wait(i);
     }
-    const double* c = Wk.read();
-    if (numiter == 1 && !(c[2 * kd] > 0)) throw Error(kErrArgument, "eigsolve: zero start vector");
     int K = have;
     double beta = 0.0;
     for (;; ++K) {
-      at(K - 1, K - 1) += c[2 * (K - have)];
-      beta = c[2 * (K - have) + 1];
+      at(K - 1, K - 1) += Wk.alpha(K - have);
+      beta = Wk.beta(K - have);
       ++numops;
       if (K == kd || beta <= tol) break;
       at(K, K - 1) = at(K - 1, K) = beta;

@@ -113,6 +113,8 @@ Context::~Context() {
   if (copy_stream) cudaStreamSynchronize(copy_stream);
   for (auto e : copy_ev)
     if (e) cudaEventDestroy(e);
+  for (auto e : krylov_ev)
+    if (e) cudaEventDestroy(e);
   if (copy_stream) cudaStreamDestroy(copy_stream);
   if (solver && solver_destroy) solver_destroy(solver);
   if (d_partials) cudaFree(d_partials);

@@ -226,8 +226,8 @@ struct Context : std::enable_shared_from_this<Context> {
   // pinned scratch, so that the host has them after any synchronisation (check_waits).
   int* wait_err = nullptr;        // [kWaitGemm], [kWaitKrylov]
   // small pinned host scratch: [0, 64) scalar results, [64, 64 + 3 * 128) the batched Lanczos
-  // and the wait_err words
-  static constexpr int kPinnedDoubles = 64 + 3 * 128 + 1;
+  // then the coefficients of a Krylov cycle, and the wait_err words
+  static constexpr int kPinnedKrylov = 64 + 3 * 128, kPinnedDoubles = kPinnedKrylov + 2 * 33 + 1;
   double* h_pinned = nullptr;
   PlanCache<DevContract> contract_cache;
   std::unordered_map<std::string, std::shared_ptr<DevReleg>> releg_cache;
@@ -238,6 +238,7 @@ struct Context : std::enable_shared_from_this<Context> {
   size_t heff_bytes = 0;
   cudaStream_t copy_stream = nullptr;   // host<->device transfers overlapped with compute
   cudaEvent_t copy_ev[4] = {};          // ... and the events that order them
+  cudaEvent_t krylov_ev[4] = {};        // ends of the last Krylov steps, created on first use
   bool counted = false;           // included in g_live_contexts
   int64_t kernel_launches = 0;    // launches of this library's kernels
   bool debug_sync = false;        // MPSG_DEBUG_SYNC=1: synchronise and check after tensor-core GEMMs
