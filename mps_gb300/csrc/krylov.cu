@@ -49,7 +49,9 @@ void small_eigh(int n, const double* A, double* evals, double* evecs) {
   }
   std::vector<int> order(n);
   for (int i = 0; i < n; ++i) order[i] = i;
-  std::sort(order.begin(), order.end(), [&](int x, int y) { return at(x, x) < at(y, y); });
+  std::sort(order.begin(), order.end(), [&](int x, int y) {  // (an order of all values: NaN last)
+    return at(x, x) < at(y, y) || (std::isnan(at(y, y)) && !std::isnan(at(x, x)));
+  });
   for (int i = 0; i < n; ++i) {
     evals[i] = at(order[i], order[i]);
     for (int k = 0; k < n; ++k) evecs[k + n * i] = v[k + n * order[i]];
