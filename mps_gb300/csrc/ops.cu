@@ -746,8 +746,11 @@ std::shared_ptr<HeffOp> heff_create(Context* ctx, const TensorMeta& vmeta, const
   op->ref_flops = applymps2site_flops(ctx, vmeta, envL.meta, envR.meta, W1.meta, W2.meta);
   op->precision = heff_arithmetic(ctx, precision, vmeta, envL.meta, envR.meta, W1.meta, W2.meta);
   if (op->precision == 0) {
-    // precision 0 reads the tensors at every application; a slice count takes them as they are now
+    // precision 0 reads the tensors at every application; a slice count takes them as they are now, once
+    // they are there
     const bool keep = precision != 0;
+    if (keep && wait_left) MPSG_CUDA(cudaStreamWaitEvent(ctx->stream, wait_left, 0));
+    if (keep && wait_right) MPSG_CUDA(cudaStreamWaitEvent(ctx->stream, wait_right, 0));
     op->envL = keep ? copy_tensor(ctx, envL) : envL;
     op->envR = keep ? copy_tensor(ctx, envR) : envR;
     op->W1 = keep ? copy_tensor(ctx, W1) : W1;
