@@ -48,6 +48,7 @@ struct DirectTables {
 
 struct DirectPlan {
   unsigned char* d_tables = nullptr;
+  size_t table_bytes = 0;
   cudaStream_t stream = nullptr;
   SmallProblem* d_small = nullptr;
   ThinUnit* d_units = nullptr;
@@ -62,6 +63,7 @@ struct DirectPlan {
   // ca, cb: A, B have imaginary parts (the products of all parts in one set of launches)
   bool build(const ContractPlan& p, const TensorMeta& A, const TensorMeta& B, int num_sms,
              cudaStream_t st, bool ca, bool cb);
+  size_t device_bytes() const { return table_bytes + (tc ? tc->table_bytes : 0); }
   ~DirectPlan();
 };
 

@@ -72,6 +72,7 @@ struct Plan {
   std::vector<Group> groups;
   cudaStream_t stream = nullptr;
   bool mapped = false;
+  size_t table_bytes = 0;  // on the device
   void build(const std::vector<Task>& g, int num_sms, cudaStream_t st);
   void release();
   double flops() const;

@@ -1244,6 +1244,7 @@ void Plan::build(const std::vector<Task>& g, int num_sms, cudaStream_t st) {
     const size_t op = img.add(t.probs), ot = img.add(t.tiles), oi = img.add(t.items),
                  oa = img.add(t.axes), ob = img.add(t.blocks);
     G.d_tables = img.upload(st);
+    table_bytes += img.bytes.size();
     G.d_probs = (Problem*)(G.d_tables + op);
     G.d_tiles = (Tile*)(G.d_tables + ot);
     G.d_items = (int2*)(G.d_tables + oi);
@@ -1264,6 +1265,7 @@ void Plan::release() {
     if (G.plain) G.plain->release();
   }
   groups.clear();
+  table_bytes = 0;
 }
 
 template <Access MAP>

@@ -415,8 +415,10 @@ bool DirectPlan::build(const ContractPlan& p, const TensorMeta& A, const TensorM
   flops = p.flops * (ca ? 2 : 1) * (cb ? 2 : 1);
   for (const auto& x : t.tiled) tc_flops += 2.0 * x.g.M * x.g.N * x.g.K;
   TableImage img;
-  const size_t os = img.add(t.small), ou = img.add(t.units), of = img.add(t.offs), ov = img.add(t.vals), oa = img.add(t.axes), ob = img.add(t.blocks);
+  const size_t os = img.add(t.small), ou = img.add(t.units), of = img.add(t.offs),
+               ov = img.add(t.vals), oa = img.add(t.axes), ob = img.add(t.blocks);
   d_tables = img.upload(st);
+  table_bytes = img.bytes.size();
   d_small = (SmallProblem*)(d_tables + os);
   d_units = (ThinUnit*)(d_tables + ou);
   d_offs = (ThinOffset*)(d_tables + of);

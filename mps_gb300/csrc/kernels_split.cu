@@ -39,6 +39,7 @@
 #include <type_traits>
 
 #include "dep_load.cuh"
+#include "f64tc.hpp"
 #include "split.hpp"
 #include "tc5.cuh"
 
@@ -856,6 +857,7 @@ size_t DevGemmPlan::device_bytes() const {
   size_t b = 0;
   for (const auto& sp : splitp)
     if (sp) b += (size_t)sp->S * (size_t)(sp->rowsA + sp->rowsB) * 128;
+  if (tc) b += tc->table_bytes;
   return b;
 }
 

@@ -139,7 +139,7 @@ struct DevGemmPlan {
   std::shared_ptr<split::SplitPlan> splitp[8];  // split-precision plans by slice count
   cudaStream_t stream = nullptr;  // tables are allocated and freed in this stream's order
   std::shared_ptr<f64tc::Plan> tc;  // the tiled tasks that run on the tensor cores (FP64)
-  size_t device_bytes() const;    // packed-slice scratch of the split plans (the bulk)
+  size_t device_bytes() const;    // packed-slice scratch of the split plans (the bulk), FP64 tables
   // num_sms > 0: the tiled tasks run on the tensor cores of that many SMs; 0 keeps every task on
   // the FP64 pipe (no scratch at launch).
   void upload(const std::vector<GemmTask>& g, double flops_, cudaStream_t st, int num_sms = 0);
@@ -159,7 +159,7 @@ struct DevContract {
   // FP64 without fused copies (null: not for this structure), by [A complex] + 2 [B complex]
   bool direct_tried[4] = {false, false, false, false};
   std::shared_ptr<DirectPlan> direct[4];
-  size_t device_bytes() const { return mm.device_bytes(); }
+  size_t device_bytes() const;         // of mm and of the index tables (16 bytes per fused index)
   ~DevContract();
 };
 
