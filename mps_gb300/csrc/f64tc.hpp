@@ -57,8 +57,8 @@ struct Group {
   int2* d_items = nullptr;
   AxisEntry* d_axes = nullptr;   // mapped groups only
   MapBlock* d_blocks = nullptr;
-  std::vector<GemmTask> tasks;
-  std::unique_ptr<DevGemmPlan> plain;  // FP64-pipe tables, built if the scratch cannot be had
+  std::vector<GemmTask> tasks;         // not of a mapped plan, whose caller has another way
+  std::unique_ptr<DevGemmPlan> plain;  // FP64-pipe tables of them, built if the scratch cannot be had
   size_t scratch_bytes() const;
 };
 

@@ -1153,7 +1153,7 @@ void plan_group(const std::vector<Task>& g, int num_sms, Group& G, GroupTables& 
         t.items.push_back(make_int2(p | (1 << 30), (int)r));
     }
     G.flops += 2.0 * x.M * x.N * x.K;
-    G.tasks.push_back(x);
+    if (!task.map) G.tasks.push_back(x);
     t.probs.push_back(P);
   }
   // Tiles of very different K, or fewer tiles than SMs, leave SMs idle: then tiles are cut along K
