@@ -60,6 +60,10 @@ int mpsg_ctx_clear_caches(mpsg_ctx* ctx);
  * MPSG_ERR_CUDA; the record is then cleared. mpsg_ctx_record_wait makes that record from a kernel on the
  * context's stream (which: 0 = FP64 product, 1 = Krylov solver), to test the callers of a program. */
 int mpsg_ctx_record_wait(mpsg_ctx* ctx, int32_t which, int32_t code);
+/* Most scratch, in bytes, that one FP64 tensor-core launch of the context may take (18 bytes per operand
+ * element; negative, the default: no limit). What needs more, or finds no memory, runs on the FP64 pipe
+ * instead, with the same accuracy and much slower. */
+int mpsg_ctx_set_scratch_limit(mpsg_ctx* ctx, int64_t bytes);
 /* Debug library only (libmpsgb300_checked.so, built with MPSG_DEVICE_CHECKS): the copy kernel
  * recomputes every block offset it decodes by plain division, checks every address against its
  * task's span, and records a violation instead of making the access (no counterpart in the

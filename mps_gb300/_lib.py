@@ -72,6 +72,7 @@ SIGNATURES = {
     "mpsg_tensor_device_ptr": [P, PP],
     "mpsg_device_checks": [P, I32, PI64, PI64],
     "mpsg_ctx_record_wait": [P, I32, I32],
+    "mpsg_ctx_set_scratch_limit": [P, I64],
     "mpsg_host_alloc": [I64, PP],
     "mpsg_host_free": [P],
     "mpsg_tensor_download_async": [P, P, P, I64, PP],

@@ -231,6 +231,13 @@ int mpsg_tensor_download(const mpsg_tensor* t, double* host, int64_t n) {
   });
 }
 
+int mpsg_ctx_set_scratch_limit(mpsg_ctx* ctx, int64_t bytes) {
+  return guarded([&] {
+    need(ctx, "ctx");
+    ctx->c.scratch_limit = bytes < 0 ? SIZE_MAX : (size_t)bytes;
+  });
+}
+
 int mpsg_ctx_record_wait(mpsg_ctx* ctx, int32_t which, int32_t code) {
   return guarded([&] {
     need(ctx, "ctx");

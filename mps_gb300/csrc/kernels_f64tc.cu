@@ -1324,7 +1324,9 @@ bool launch(Context* ctx, Plan& p, const double* A, const double* B, double* C,
   for (Group& G : p.groups) {
     if (G.ntiles == 0) continue;
     unsigned char* mem = nullptr;
-    const cudaError_t e = cudaMallocAsync((void**)&mem, G.scratch_bytes(), st);
+    const size_t need = G.scratch_bytes();
+    const cudaError_t e = need > ctx->scratch_limit ? cudaErrorMemoryAllocation
+                                                    : cudaMallocAsync((void**)&mem, need, st);
     if (e == cudaErrorMemoryAllocation) {
       // no room for the packed operands (twice the FP64 ones): the FP64-pipe kernel needs none
       (void)cudaGetLastError();

@@ -240,6 +240,7 @@ struct Context : std::enable_shared_from_this<Context> {
   cudaEvent_t copy_ev[4] = {};          // ... and the events that order them
   cudaEvent_t krylov_ev[4] = {};        // ends of the last Krylov steps, created on first use
   bool counted = false;           // included in g_live_contexts
+  size_t scratch_limit = SIZE_MAX;  // of one FP64 tensor-core launch; what needs more takes the FP64 pipe
   int64_t kernel_launches = 0;    // launches of this library's kernels
   bool debug_sync = false;        // MPSG_DEBUG_SYNC=1: synchronise and check after tensor-core GEMMs
   double gemm_flops = 0;          // algorithmic flops issued through block GEMMs
