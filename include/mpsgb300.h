@@ -16,8 +16,8 @@
  *     (column-major sector order, last leg slowest, src/sector.jl:35-36), each block
  *     column-major, blocks concatenated (mpsg_tensor_sectors gives the offsets).
  *   - `precision` selects the block-GEMM arithmetic: 0 = FP64 (the plain drop-in; on the tensor
- *     cores as 9-bit digits, every element of a result at least as accurate as a sum of FP64 FMAs
- *     guarantees: within K 2^-53 of sum |a b|); s = 2..7 = at least the accuracy of split precision with
+ *     cores as 9-bit digits, no element of a result less accurate than sums of K FP64 FMAs are, and
+ *     within K 2^-51 of sum |a b| at worst); s = 2..7 = at least the accuracy of split precision with
  *     s bf16 slices per operand, FP32 accumulation in tensor memory and an FP64 epilogue. Where FP64
  *     is the faster arithmetic (s >= 6, and contractions up to about 20 GFLOP) it is what runs.
  *   - All work is ordered on the context's CUDA stream; calls that return host values

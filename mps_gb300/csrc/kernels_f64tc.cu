@@ -22,12 +22,11 @@
 //     kWideK; longer K is cut into pieces) and the others into a second one (unit 2^-63, or FP32).
 //     At the end both are rounded to FP64 once. No FP64 instruction is issued.
 //
-// Accuracy, element by element: what a mode leaves out is below 2^-53 of sum |a b| rms and, at worst, below
-// the bound of a chain of K FP64 FMAs, K 2^-53 sum |a b| (mode_of), so no element is less accurate than
-// FP64 arithmetic makes it, however its operands are graded. An element for which that cannot be shown
-// is computed by FP64 FMAs (fma_element). For operands of one size the result is rounded once, where the chain
-// rounds K times: relative error of N(0,1) products against extended precision 2e-16 (K = 33) to 1.4e-15
-// (K = 2050) on the FP64 pipe, 5e-17 here.
+// Accuracy, element by element, however the operands are graded (mode_of): what is left out is below 2^-53
+// of sum |a b| rms, or below what a chain of K FP64 FMAs rounds rms, and at most K 2^-51 of sum |a b|; an
+// element for which that cannot be shown is computed by FP64 FMAs (fma_element). For operands of one size the
+// result is rounded once, where the chain rounds K times: relative error of N(0,1) products against
+// extended precision 2e-16 (K = 33) to 1.4e-15 (K = 2050) on the FP64 pipe, 5e-17 here.
 //
 // A row with a non-finite element, or whose largest element is outside 2^-400..2^400, is marked
 // in its exponent; every output element of such a row or column is computed in the epilogue by
@@ -43,11 +42,11 @@
 // Measured: one 4096 x 4000 x 4096 product 3.3 ms (40 TFLOP/s of FP64 work; the FP64 pipe takes 125 ms).
 // Before the MMAs were issued from code that the whole warp runs in step (elect_one) they took 80 cycles
 // each, most of them to move their operands to uniform registers. A two-site H_eff (packing, this
-// kernel, two thin steps, packing, this kernel) takes 573 us at chi = 2048 (9680 on the FP64 pipe) and
-// 95 us at chi = 517 (1005). Seven digits and no bound for the elements, as 128 x 80 tiles, took 522 and 90
+// kernel, two thin steps, packing, this kernel) takes 574 us at chi = 2048 (9680 on the FP64 pipe) and
+// 96 us at chi = 517 (1005). Seven digits and no bound for the elements, as 128 x 80 tiles, took 522 and 90
 // us, and lost all digits of a small element next to a large one. The same with every element of the
-// tensors scaled by a power of ten of its own, over 3, 8, 16 decades: 807, 814, 923 us at chi = 2048,
-// 110, 123, 205 at chi = 517.
+// tensors scaled by a power of ten of its own, over 3, 8, 16 decades: 774, 782, 827 us at chi = 2048,
+// 113, 115, 162 at chi = 517.
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 
@@ -87,7 +86,7 @@ struct Digits {
 // such a stretch.
 template <int MODE>
 __device__ __forceinline__ constexpr int drain_steps(int g) {
-  return g == 0 ? 32 : g == 1 ? 8 : g == 2 ? 4 : g <= 4 ? 2 : MODE != kAll ? 32 : g == 7 ? 8 : 1;
+  return g == 0 ? 32 : g == 1 ? 8 : g == 2 ? 4 : g <= 4 ? 2 : MODE != kAll ? 32 : 1;
 }
 template <int MODE>
 __device__ __forceinline__ bool drain_begin(int g, int ks) {
@@ -100,16 +99,20 @@ __device__ __forceinline__ bool drain_end(int g, int ks, int nk) {
 constexpr int kABytes = BM * BK * 2, kBBytes = BN * BK * 2;
 constexpr int kStageBytes = kSlices * (kABytes + kBBytes);  // 108 KB
 constexpr int kStages = 2;
-constexpr int kSmemBytes = kStages * kStageBytes + 1024 + 256;  // (barriers and a few words: 224)
+constexpr int kSmemBytes = kStages * kStageBytes + 1024 + 256 + BM * BN / 8;  // (barriers, words: 224)
 constexpr int kTmemCols = 512;
 static_assert(kAccs * BN <= kTmemCols, "accumulators fit TMEM");
 constexpr int kEpiWarps = 16;
 constexpr int kThreads = 32 * (2 + kEpiWarps);
 constexpr int kEpiCols = BN * 4 / kEpiWarps;  // 16 columns per epilogue thread
+static_assert(kEpiWarps == 16 && kEpiCols == 16, "finish_tile shares out columns modulo 16");
 
-constexpr int kRowZero = 1 << 20;  // exponent entry of an all-zero row
-constexpr int kRowBad = 1 << 21;   // ... of a row outside the sliced range (see above)
 constexpr int kExpRange = 400;
+// A row's entry: its exponent << kCountBits | its number of middling elements (see mode_of), K at most.
+constexpr int kCountBits = 17, kCountMask = (1 << kCountBits) - 1;
+constexpr int kRowZero = 1000;  // exponent of an all-zero row
+constexpr int kRowBad = 1001;   // ... of a row outside the sliced range (see above)
+static_assert(kMaxK <= kCountMask && kExpRange < kRowZero, "counts and exponents fit an entry");
 constexpr int kRowBlock = 32;      // rows per packing item
 static_assert(BM % kRowBlock == 0 && BN % kRowBlock == 0, "a row block is in one tile");
 
@@ -120,13 +123,20 @@ static_assert(BM % kRowBlock == 0 && BN % kRowBlock == 0, "a row block is in one
 //   kFew   sqrt(K) 2^-61.3 RR rms, at most K 2^-58.4 RR (the products of weight 2^-63),
 //   kMore  sqrt(K) 2^-65.6 RR rms, at most K 2^-61 RR (the rounding of the elements),
 // each taken where that is below 2^-53 S rms and, at worst, below the worst case of the FMA chain,
-// K 2^-53 S. kAll leaves out K 2^-74 RR at most, which does for outputs |y| >= 2^-kGuardBits RR; the
-// others are computed again by FP64 FMAs. N(0,1) operands pass the first from K of about 60 on, and so
-// does the MPO-contracted intermediate of an XXZ H_eff, a sixth of it zeros: 97% of the work at
-// chi = 517, 99% at chi = 1024; the last contraction of environment updates 91% and, all but edge charges,
-// the second.
+// K 2^-53 S. kAll leaves out sqrt(K) 2^-79 RR rms, K 2^-75 RR at most. The FMA chain's rounding is about
+// 0.4 sqrt(K) 2^-53 S rms where the terms have one sign and 2^-54.5 S where the signs are random, |y| being
+// about S and S / sqrt(K) then: in both cases no less than kAll's at |y| = 2^-kGuardBits RR. Smaller outputs are
+// computed again by FP64 FMAs, unless their row and column have n >= sqrt(K / 2) elements from 2^-kMidBits of
+// their bounds on at the same k (counted likewise; S >= n 2^-24 RR).
+// N(0,1) operands pass the first from K of about 60 on, and so does the MPO-contracted intermediate of an XXZ
+// H_eff, a sixth of it zeros: 97% of the work at chi = 517, 99% at chi = 1024; the last contraction of
+// environment updates 91% and, all but edge charges, the second. Real states are graded: 9 in 10 tiles of a
+// chi = 2048 sweep's environments take all digits, and 1.6 million of their 1.2e9 elements FMAs (16
+// million with 2^-20 for the guard and no count of middling elements; the sweep's FP64 products take 197 ms
+// so, 757 then, 120 with no FMAs, 93 with seven digits and no bound).
 constexpr int kLargeBits = 5;
-constexpr int kGuardBits = 20;
+constexpr int kMidBits = 12;
+constexpr int kGuardBits = 24;
 
 __device__ __forceinline__ int mode_of(int la, int lb, int64_t K) {
   const int64_t n = (int64_t)la + lb - K;
@@ -380,7 +390,7 @@ __global__ void __launch_bounds__(256, 4) pack_f64_kernel(
   extern __shared__ double xs[];  // [k][row], rows padded to kPadRows
   __shared__ uint32_t red[8][33], rlow[8][33];  // largest high words, all low words or-ed
   __shared__ uint2 rmax[kRowBlock];
-  __shared__ int rexp[kRowBlock], large[kRowBlock];  // large: large elements of a row
+  __shared__ int rexp[kRowBlock], large[kRowBlock], mid[kRowBlock];  // mode_of's counts
   cudaTriggerProgrammaticLaunchCompletion();
   const int t = threadIdx.x, lane = t & 31, w = t >> 5;
   const int rank = blockIdx.x % ncta;
@@ -465,7 +475,7 @@ __global__ void __launch_bounds__(256, 4) pack_f64_kernel(
       lo |= rlow[g][t];
     }
     rmax[t] = make_uint2(m, lo);
-    large[t] = 0;
+    large[t] = mid[t] = 0;
   }
   if (ncta > 1) cg::this_cluster().sync();
   else __syncthreads();
@@ -479,15 +489,14 @@ __global__ void __launch_bounds__(256, 4) pack_f64_kernel(
     if ((m.x | m.y) == 0) e = kRowZero;
     else if (e < -kExpRange || e > kExpRange) e = kRowBad;  // also Inf and NaN
     rexp[t] = e;
-    if (rank == 0 && t < nr) (side ? RB + P.rB : RA + P.rA)[r0 + t] = e;
   }
   __syncthreads();
   // digits: a warp covers 4 rows x 32 K of one step, a thread 4 consecutive K of a row (with 8 it takes
   // 80 registers, three CTAs per SM instead of four)
   constexpr int kPer = 4;
   const int rr = w * 4 + (lane & 3), g4 = (lane >> 2) * kPer;  // (no bank conflicts so)
-  const int e = rexp[rr];
-  int nlarge = 0;
+  const int e = rexp[rr] < kRowZero ? rexp[rr] : 1 << 20;
+  int counts = 0;  // large elements | middling ones << 16 (of 8 threads: at most 8192)
   if (rr < nr) {
     const int rpt = side ? BN : BM;
     const int64_t r = r0 + rr;
@@ -517,7 +526,7 @@ __global__ void __launch_bounds__(256, 4) pack_f64_kernel(
         // at 63 and d >= 0 the distance to the row's largest exponent (nothing is left of zeros,
         // subnormals and the elements of a row that is not sliced), and its complement if x < 0
         const int d = e + 1022 - (int)((hw >> 20) & 0x7ffu);
-        nlarge += d < kLargeBits;
+        counts += (d < kLargeBits) + ((d < kMidBits) << 16);
         const uint32_t m1 = __funnelshift_l(lw, hw, 11) | 0x80000000u, m0 = lw << 11;
         uint32_t f0, f1, f2;
         if (d < 16) {
@@ -564,9 +573,12 @@ __global__ void __launch_bounds__(256, 4) pack_f64_kernel(
     }
   }
   // the fewest large elements of a row, over the rows that the digits stand for
-  for (int o = 4; o < 32; o <<= 1) nlarge += __shfl_xor_sync(0xffffffffu, nlarge, o);
-  if (lane < 4 && nlarge)
-    atomicAdd(ncta > 1 ? cg::this_cluster().map_shared_rank(&large[rr], 0) : &large[rr], nlarge);
+  for (int o = 4; o < 32; o <<= 1) counts += __shfl_xor_sync(0xffffffffu, counts, o);
+  if (lane < 4 && counts) {
+    const auto cl = cg::this_cluster();
+    atomicAdd(ncta > 1 ? cl.map_shared_rank(&large[rr], 0) : &large[rr], counts & 0xffff);
+    atomicAdd(ncta > 1 ? cl.map_shared_rank(&mid[rr], 0) : &mid[rr], counts >> 16);
+  }
   // (nor does a CTA leave before the others have read its maxima)
   if (ncta > 1) cg::this_cluster().sync();
   else __syncthreads();
@@ -574,6 +586,8 @@ __global__ void __launch_bounds__(256, 4) pack_f64_kernel(
     const bool sliced = lane < nr && rexp[lane] < kRowZero;
     const int least = __reduce_min_sync(0xffffffffu, sliced ? large[lane] : (int)K);
     if (lane == 0) (side ? LB + P.lB : LA + P.lA)[r0 / kRowBlock] = least;
+    if (lane < nr)
+      (side ? RB + P.rB : RA + P.rA)[r0 + lane] = rexp[lane] * (kCountMask + 1) + (sliced ? mid[lane] : 0);
   }
 }
 
@@ -588,7 +602,7 @@ __device__ __noinline__ void fma_chains(const Problem& P, int64_t row, int64_t n
   Cursor<MAP> out(blocks + P.blkC, m_ax, P.oc, row, P.crs, MAP ? P.nnc : P.ccs,
                   parts.c1, parts.c2, parts.c3);
   for (int j = 0; j < nc; ++j) {
-    if (!all && RB[j] != kRowBad) continue;
+    if (!all && RB[j] >> kCountBits != kRowBad) continue;
     Cursor<MAP> a(blocks + P.blkA, m_ax, P.oa, row, P.ars, MAP ? P.nkc : P.aks,
                   P.swap ? parts.b : parts.a);
     Cursor<MAP> b(blocks + P.blkB, n_ax + n0 + j, P.ob, n0 + j, P.brs, MAP ? P.nkc : P.bks,
@@ -703,6 +717,8 @@ __device__ __forceinline__ bool drain_tile(int nk, uint32_t taddr, uint64_t* tfu
   return true;
 }
 
+constexpr int kRedoAt = 10;
+
 // What the epilogue of a tile works with.
 struct Epilogue {
   uint64_t *tfull, *tempty, *esync;
@@ -786,21 +802,24 @@ __device__ __forceinline__ bool finish_tile(const Epilogue& e, const Tile& tr, c
   const double *R = P.swap ? e.B : e.A, *S = P.swap ? e.A : e.B;
   uint32_t redo = 0;  // columns of this row that are left to FMAs
   if (row < P.M) {
-    const int er = K ? e.RA[P.rA + row] : kRowZero;
+    const int ra = K ? e.RA[P.rA + row] : kRowZero << kCountBits, er = ra >> kCountBits;
     const int32_t* RBp = e.RB + P.rB + n0;
     bool bad = er == kRowBad;
 #pragma unroll
     for (int j = 0; j < kEpiCols; ++j) {  // the sums' registers take the FP64 bits
-      const int ec = K && j < nc ? RBp[j] : kRowZero;
+      const int rb = K && j < nc ? RBp[j] : kRowZero << kCountBits, ec = rb >> kCountBits;
       bad = bad || ec == kRowBad;
       const double y =
           er >= kRowZero || ec >= kRowZero
               ? 0.0
               : sum_to_f64(hi[j], lo[j], wide ? kHiUnit - kWideShift : kHiUnit, er + ec - 14);
       hi[j] = __double_as_longlong(y);
-      if constexpr (ALL) {  // |y| < 2^(er + ec - kGuardBits), by the high word
+      if constexpr (ALL) {  // |y| < 2^(er + ec - kGuardBits), by the high word, and too few middling terms
         const int limit = (er + ec - kGuardBits + 1023) << 20;
-        if (er < kRowZero && ec < kRowZero && (__double2hiint(y) & 0x7fffffff) < limit) redo |= 1u << j;
+        const int n = (ra & kCountMask) + (rb & kCountMask) - K;
+        if (er < kRowZero && ec < kRowZero && (__double2hiint(y) & 0x7fffffff) < limit &&
+            (n < 1 || 2 * (int64_t)n * n < K))
+          redo |= 1u << j;
       }
     }
     Cursor<MAP> out(e.blocks + P.blkC, e.axes + P.axM + row, P.oc, row, P.crs, MAP ? P.nnc : P.ccs,
@@ -815,12 +834,30 @@ __device__ __forceinline__ bool finish_tile(const Epilogue& e, const Tile& tr, c
       fma_chains<MAP>(P, row, n0, nc, er == kRowBad, RBp, e.axes, e.blocks, R, S, e.C, parts);
   }
   if constexpr (ALL) {
-    __syncwarp();
-    for (uint32_t rows = __ballot_sync(0xffffffffu, redo != 0); rows; rows &= rows - 1) {
-      const int from = __ffs(rows) - 1;
-      for (uint32_t cols = __shfl_sync(0xffffffffu, redo, from); cols; cols &= cols - 1)
-        fma_element<MAP>(P, row - lane + from, n0 + __ffs(cols) - 1, e.axes, e.blocks, R, S, e.C, parts);
+    // The elements left to FMAs are often those of a few rows or columns: every warp takes those of one
+    // diagonal, modulo 16 (with its own rows and columns for each warp, the FP64 products of a chi = 2048
+    // sweep's environments and energies take 294 ms instead of 197).
+    volatile uint16_t* bits = (volatile uint16_t*)(e.last_part + kRedoAt);  // [tile row][16 columns]
+    bits[lrow * 4 + (col0 >> 4)] = (uint16_t)redo;
+    mbar_arrive(e.esync);
+    if (!__all_sync(0xffffffffu, mbar_wait(e.esync, 0, e.abort_flag, e.err, 6))) return false;
+    const int rows = (int)min((int64_t)BM, P.M - (int64_t)tr.mi * BM);
+    for (int r0 = 0; r0 < rows; r0 += 32) {  // a row per lane, then the rows that have such elements
+      const int r = r0 + lane, c = (warp - 2 + r) & 15;
+      uint32_t which = 0;
+#pragma unroll
+      for (int j = 0; j < BN / 16; ++j)
+        which |= (uint32_t)(r < rows ? bits[r * 4 + j] >> c & 1 : 0) << j;
+      for (uint32_t todo = __ballot_sync(0xffffffffu, which != 0); todo; todo &= todo - 1) {
+        const int l = __ffs(todo) - 1;
+        for (uint32_t q = __shfl_sync(0xffffffffu, which, l); q; q &= q - 1)
+          fma_element<MAP>(P, (int64_t)tr.mi * BM + r0 + l,
+                           (int64_t)tr.ni * BN + 16 * (__ffs(q) - 1) + ((warp - 2 + r0 + l) & 15), e.axes,
+                           e.blocks, R, S, e.C, parts);
+      }
     }
+    mbar_arrive(e.esync);  // the next such tile writes the masks again
+    if (!__all_sync(0xffffffffu, mbar_wait(e.esync, 1, e.abort_flag, e.err, 6))) return false;
   }
   return true;
 }
@@ -863,6 +900,7 @@ __global__ void __launch_bounds__(kThreads, 1) gemm_f64tc_kernel(
   // K steps. It is at most two tiles ahead, as it waits for the accumulators of the one before.
   constexpr int kInfo = 4;
   volatile uint32_t* info = tmem_slot + 3;
+  // ... and after it, kRedoAt words from last_part on, a bit per output element (finish_tile)
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {

@@ -235,7 +235,7 @@ DeviceTensor symmatrix(Context* ctx, const DeviceTensor& a, const std::vector<in
 // block GEMM dispatch
 // ------------------------------------------------------------------------------------------
 // The arithmetic that a precision argument runs with: from 6 slices on the FP64 products of the
-// tensor cores (9-bit digits, 28 to 45 products, no element less accurate than FP64 FMAs make it), where the 6-
+// tensor cores (9-bit digits, 28 to 45 products, no element less accurate than FP64 FMAs are), where the 6-
 // and 7-slice split products take 21 and 28 and passes of their own for 1e-12 and 1e-14.
 static int arithmetic(int precision) {
   if (precision == 0 || (precision >= 2 && precision < kFp64Slices)) return precision;
