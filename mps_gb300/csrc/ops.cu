@@ -318,20 +318,15 @@ static void ensure_fused(Context* ctx, DevContract& p) {
   p.fused = true;
 }
 
-size_t DevContract::device_bytes() const {
-  size_t b = mm.device_bytes();
-  for (const auto& d : direct)
-    if (d) b += d->device_bytes();
-  return b;
-}
-
 static DirectPlan* direct_plan(Context* ctx, DevContract& p, bool ca = false, bool cb = false) {
   const int i = (ca ? 1 : 0) + (cb ? 2 : 0);
   if (!p.direct_tried[i]) {
     auto d = std::make_shared<DirectPlan>();
-    if (d->build(*p.host, p.metaA, p.metaB, ctx->num_sms, ctx->stream, ca, cb)) p.direct[i] = d;
+    if (d->build(*p.host, p.metaA, p.metaB, ctx->num_sms, ctx->stream, ca, cb)) {
+      p.direct[i] = d;
+      p.direct_bytes += d->device_bytes();
+    }
     p.direct_tried[i] = true;
-    ctx->contract_cache.trim();  // (never evicts the entry in use, which is the latest)
   }
   return p.direct[i].get();
 }

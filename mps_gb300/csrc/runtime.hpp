@@ -159,7 +159,8 @@ struct DevContract {
   // FP64 without fused copies (null: not for this structure), by [A complex] + 2 [B complex]
   bool direct_tried[4] = {false, false, false, false};
   std::shared_ptr<DirectPlan> direct[4];
-  size_t device_bytes() const;         // of mm and of the index tables (16 bytes per fused index)
+  size_t direct_bytes = 0;             // their tables (16 bytes per fused index)
+  size_t device_bytes() const { return mm.device_bytes() + direct_bytes; }
   ~DevContract();
 };
 
