@@ -275,8 +275,10 @@ int mpsg_plan_contract_tasks(const mpsg_tensor* a, const int32_t* idxa, const mp
 /* ---- prepared two-site effective Hamiltonian ---------------------------------------------- */
 /* The matvec closure v -> _applymps2site(v, envL, envR, W1, W2) of src/dmrg.jl:77 as an object
  * that is built once per bond and applied many times.  precision 0 runs the reference's four
- * FP64 contractions; precision S >= 2 folds W1 into envL and W2 into envR once and applies
- * H_eff as two split-precision tensor-core GEMMs whose constant operands are sliced once. */
+ * FP64 contractions on the tensors as they are at each application; precision S = 2..4, and 5 from
+ * 4 GFLOP on, folds W1 into envL and W2 into envR once and applies H_eff as two split-precision
+ * tensor-core GEMMs whose constant operands are sliced once. S = 6 and 7, and 5 below 4 GFLOP, runs the
+ * four FP64 contractions, which are faster there, on copies of the four tensors made at creation. */
 typedef struct mpsg_heff mpsg_heff;
 int mpsg_heff2_create(mpsg_ctx* ctx, const mpsg_tensor* v_like, const mpsg_tensor* envl,
                       const mpsg_tensor* envr, const mpsg_tensor* w1, const mpsg_tensor* w2,
@@ -286,7 +288,8 @@ int mpsg_heff2_apply(mpsg_ctx* ctx, mpsg_heff* op, const mpsg_tensor* v, mpsg_te
 int mpsg_heff2_flops(const mpsg_heff* op, double* flops);
 /* Algorithmic bytes per application of a prepared split-precision operator: block-permute
  * copies (8 read + 8 written per element moved) and operand packing (exponent pass 8 read, slice
- * pass 8 read + 2 S written per element); 0 for precision 0. For HBM rooflines of those kernels. */
+ * pass 8 read + 2 S written per element); 0 for an operator that runs FP64 (above). For HBM rooflines of
+ * those kernels. */
 int mpsg_heff2_traffic(const mpsg_heff* op, double* copy_bytes, double* pack_bytes);
 int mpsg_heff2_free(mpsg_heff* op);
 

@@ -37,7 +37,7 @@ namespace {
 constexpr int kLanes = 8;  // solver lanes created per context; MPSG_SOLVER_LANES of them used
 
 // Lanes a call spreads its blocks over: MPSG_SOLVER_LANES (1..8), default all. The density-matrix
-// truncation of a chi = 1024 two-site tensor (17 blocks) takes 77, 48, 31 ms on 1, 4, 8 lanes (33 on 16).
+// truncation of a chi = 1024 two-site tensor (17 blocks) takes 77, 48, 30 ms on 1, 4, 8 lanes (33 on 16).
 int active_lanes() {
   const char* e = std::getenv("MPSG_SOLVER_LANES");
   const int n = e ? std::atoi(e) : kLanes;

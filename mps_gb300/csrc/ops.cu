@@ -245,8 +245,8 @@ static int arithmetic(int precision) {
 
 // Fewer slices pay only where MMAs are what takes the time. A split contraction fuses and packs its
 // operands and pads the MPO steps to whole tiles, none of which the FP64 contraction in place does: a
-// left environment update in us, FP64 / 4 / 5 slices: chi = 96 35 / 225 / 236, chi = 1024 140 / 596 /
-// 661, chi = 2048 327 / 1448 / 1684. So up to this many flops in the sector GEMMs that are not thin (a
+// left environment update in us, FP64 / 4 / 5 slices: chi = 96 13 / 225 / 236, chi = 1024 142 / 596 /
+// 661, chi = 2048 383 / 1448 / 1684. So up to this many flops in the sector GEMMs that are not thin (a
 // few times the largest contraction of those updates, where 5 slices would save 0.3 ms of MMAs)
 // a contraction asked for with slices gets FP64 results.
 constexpr double kSplitContractFlops = 2e10;
@@ -450,12 +450,14 @@ static const std::vector<int> kH2A = {1, -1, -2, 4, 5}, kH2B = {-1, 2, 3, -2};
 static const std::vector<int> kH3A = {1, 2, -1, -2, 5}, kH3B = {-1, 3, 4, -2};
 static const std::vector<int> kH4A = {1, 2, 3, -1, -2}, kH4B = {-2, -1, 4};
 
-// The arithmetic of a two-site H_eff. Five slices pay from about 4 GFLOP on, where the MMAs that they save
-// outweigh their extra passes (fused copies, exponents, W folded into the environments): FP64 / 5
-// slices in us, chi = 48 17 / 101, 517 106 / 172, 1024 194 / 254, 1448 330 / 334, 2048 549 / 466 (since
-// then both faster by 5%, 521 / 442).
-// Smaller operators asked for with five slices get FP64 results. (Fewer slices are kept at every
-// size: a batch runs slices, and its operators agree with single ones to rounding there.)
+// The arithmetic of a prepared two-site H_eff. Five slices pay from about 4 GFLOP on, where the MMAs that
+// they save outweigh their extra passes (fused copies, exponents, W folded into the environments): FP64 / 5
+// slices in us, chi = 48 17 / 95, 517 102 / 163, 1024 212 / 233, 1200 257 / 260, 1448 (4.0 GFLOP) 322 / 316,
+// 1700 435 / 367, 2048 576 / 443. Smaller operators asked for with five slices get FP64 results, which
+// a batch, which runs slices at every size, does not give them: the two agree to the slicing error
+// (1.6e-10) there. Two to four slices run as slices at every size, and agree with a batch to rounding; that is
+// the slower and less accurate choice below about 1.5 GFLOP (FP64 / 2 / 3 / 4 slices in us, chi = 517 102 /
+// 160 / 175 / 146, 1024 216 / 188 / 223 / 193, 2048 575 / 335 / 392 / 363).
 constexpr double kHeffFp64Flops = 4e9;
 
 static int heff_arithmetic(Context* ctx, int precision, const TensorMeta& v, const TensorMeta& envL,
@@ -467,8 +469,8 @@ static int heff_arithmetic(Context* ctx, int precision, const TensorMeta& v, con
 }
 
 // ... and of a single application, which with slices also folds W into the environments and slices the
-// result, us, 3 / 4 / 5 slices and FP64: chi = 517 285 / 249 / 172 / 108, 2048 769 / 740 / 838 / 567,
-// 2900 (23 GFLOP) 1176 / 1242 / 1524 / 1119, 4096 (58 GFLOP) 2012 / 2256 / 2832 / 2249.
+// result, us, 3 / 4 / 5 slices and FP64: chi = 517 285 / 249 / 172 / 103, 2048 769 / 740 / 838 / 577,
+// 2900 (23 GFLOP) 1182 / 1256 / 1533 / 1162, 4096 (58 GFLOP) 2021 / 2274 / 2855 / 2332.
 // Up to kSplitContractFlops it gets FP64 results for any slice count.
 static int single_arithmetic(Context* ctx, int precision, const TensorMeta& v, const TensorMeta& envL,
                              const TensorMeta& envR, const TensorMeta& W1, const TensorMeta& W2) {

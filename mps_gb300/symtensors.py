@@ -6,7 +6,10 @@ operation runs as CUDA kernels of ``libmpsgb300.so``.  The only host work is boo
 metadata and copying flat arrays in or out.
 
 ``precision`` arguments select the block-GEMM arithmetic: 0 = FP64 (the reference's Float64
-path), s >= 2 = split precision with s bf16 slices (FP32 accumulation, FP64 epilogue).
+path), s = 2..7 = at least the accuracy of split precision with s bf16 slices (FP32 accumulation,
+FP64 epilogue). Where FP64 is the faster arithmetic it is what runs: for 6 and 7 slices everywhere but
+in batches, for fewer in contractions and single applications up to about 20 GFLOP and, with five
+slices, in prepared operators below 4 GFLOP.
 """
 from __future__ import annotations
 
@@ -642,8 +645,9 @@ def applymps2site(v, envL, envR, W1, W2, precision=None) -> SymTensor:
 class Heff2:
     """The two-site effective Hamiltonian v -> _applymps2site(v, envL, envR, W1, W2)
     (src/apply.jl:93-105) prepared once and applied many times, as the Krylov solver does
-    (src/dmrg.jl:77).  ``precision`` 0 = the reference's FP64 contractions; S >= 2 = W-folded
-    split-precision tensor-core path."""
+    (src/dmrg.jl:77).  ``precision`` 0 = the reference's FP64 contractions, which read the tensors
+    at every application; S = 2..4, and 5 from 4 GFLOP on = W-folded split-precision tensor-core path; S = 6
+    and 7, and 5 below = the FP64 contractions on copies of the tensors as they are now."""
 
     def __init__(self, v_like, envL, envR, W1, W2, precision=None):
         h = C.c_void_p()

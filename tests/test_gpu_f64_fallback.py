@@ -83,3 +83,15 @@ def test_longest_contracted_index(k, packed):
                                                       precision=0))
     assert (packs > 0) == packed
     check(got, a, b)
+
+
+@pytest.mark.parametrize("m,n", [(63, 127), (64, 128), (65, 129), (127, 63), (128, 64), (129, 65), (257, 33),
+                                 (33, 257)])
+@pytest.mark.parametrize("k", [33, 96])
+def test_tile_edges(m, n, k):
+    """Both sides of the 128 x 64 tile, either operand on the long one."""
+    rng = np.random.default_rng(4)
+    a, b = rng.standard_normal((m, k)), rng.standard_normal((k, n))
+    check(mg.matmul(up(a, sp(m), mg.dual(sp(k))), up(b, sp(k), mg.dual(sp(n))), precision=0), a, b)
+    A = up(a.reshape((m, k, 1), order="F"), sp(m), mg.dual(sp(k)), sp(1))
+    check(mg.contract(A, (1, -1, 3), up(b, sp(k), mg.dual(sp(n))), (-1, 2), precision=0), a, b)
