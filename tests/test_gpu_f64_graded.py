@@ -7,7 +7,8 @@ element, S = sum |a b| and n the number of k at which both elements are surely l
 power of two): rounding the result 1.07 u |y|, and what is left out,
   K 2^-58.4 RR   with 28 products of digits (n >= 25 and n >= 3.24 sqrt(K) only),
   K 2^-60.9 RR   with 34 (n >= 4 and n >= sqrt(K) / 6 only),
-  K 2^-74 RR     with 45, for |y| >= 2^-20 RR; (K / 32 + 6) u S for the others, sums of FP64 FMAs."""
+  K 2^-74 RR     with 45, for |y| >= 2^-20 RR; (K / 32 + 6) u S for the others, which are sums of FP64 FMAs
+                 or shown to be no further off."""
 import numpy as np
 import pytest
 
